@@ -1,5 +1,5 @@
 // Shared definitions of libdnlgpu: element traits, device-side time state, kernel argument packs
-// and the handle.  All arithmetic is FP64.
+// and the handle.  State and results are FP64.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "dnl_gpu.h"
+#include "dnl_ff.cuh"
 
 namespace dnl {
 
@@ -215,6 +216,7 @@ struct Material {
   double dfun0;      // Sqrt32 * 2.0 * G, first term of dfun      (Element.C:309)
   double Cs;         // Courant sound speed with the mean nodal density (Element.C:607-621)
   double rG3;        // 1 / (3 G), for the first radial-return guess (Element.C:298)
+  MatFF f;           // the same as FP32 pairs
   HardLaw hard;
 };
 
@@ -242,6 +244,7 @@ inline Material make_material(const dnl_material &mt, int nen = 4)
   ro /= nen;
   const double Nu = m.nu;
   m.Cs = sqrt((m.young * (1 - Nu)) / (ro * (1 + Nu) * (1 - 2 * Nu)));
+  m.f = make_mat_ff(m.G2, m.G3, m.K, m.A, m.B, m.n, m.dfun0, m.rho * m.Cs);
   m.hard.law = DNL_HARD_POWER;
   m.hard.tabN = 0;
   m.hard.tab = nullptr;

@@ -1,4 +1,4 @@
-// Element kernels of libdnlgpu (sm_103a, FP64).
+// Element kernels of libdnlgpu (sm_103a).
 //
 // k_elem<ET>   one pass of Domain::computeInternalMatrices + Domain::computeInternalForces:
 //              per integration point the shape-function gradients (Element2D.C:53-126,
@@ -10,21 +10,23 @@
 // k_courant    ElQua4nAx::getLength (ElQua4nAx.C:131-143) or the tetrahedra's shortest edge
 //              (ElTet4n3D.C:151-166) over Element::getSoundSpeed, min-reduced (Domain.C:1613-1646).
 //
+// Two forms of the pass: in pairs of FP32 numbers for small increments (elem_fast,
+// dnl_elem_ff.cuh: nearly every point of every step), and in FP64 (elem_ip below) for the rest and
+// for the 10-node tetrahedron; elem_point picks per element.
+//
 // Threading: one thread per integration point; the NIP threads of an element are adjacent lanes
 // of one warp (32 % NIP == 0), so the element-mean pressure and the force sum over integration
-// points are warp-local (shuffles and a per-warp shared-memory transpose), and the
-// integration-point state, stored component-major, is read and written with coalesced accesses.
-// Where an element has more nodes than integration points (the tetrahedra), lane pt assembles
-// nodes pt, pt + NIP, ...
+// points are warp-local (shuffles and per-warp shared memory), and the integration-point state,
+// stored component-major, is read and written with coalesced accesses.
 //
-// Rounding: GB300 executes FP64 at a small fraction of its other rates, so the kernels are written
-// to minimise FP64 instructions with explicit fused multiply-adds (this file is compiled with
-// -fmad=false: the compiler fuses nothing by itself, so every instantiation of the element code --
-// single mesh, batch, tape, caller-allocated -- rounds identically) -- except in C = F^T F, which
-// uses __dmul_rn/__dadd_rn in the reference's association order (F itself is formed as
-// I + G_u J^-1, its diagonal sums added to 1 last); the Jacobi rotations then move the eigenvalues
-// by a few ulps of 1 against the reference's (see jacobi_rotate).  Elsewhere results differ from
-// the reference by a few units in the last place; the parity tests hold them to 1e-12 per pass.
+// Rounding: this file is compiled with -fmad=false (the compiler fuses nothing by itself), so every
+// instantiation of the element code -- single mesh, batch, tape, caller-allocated -- rounds
+// identically.  The FP64 pass is written to minimise FP64 instructions (64 cycles each per warp and
+// scheduler) with explicit fused multiply-adds -- except in C = F^T F, which uses
+// __dmul_rn/__dadd_rn in the reference's association order (F itself is formed as I + G_u J^-1, its
+// diagonal sums added to 1 last); the Jacobi rotations then move the eigenvalues by a few ulps of 1
+// against the reference's (see jacobi_rotate).  Elsewhere results differ from the reference by a
+// few units in the last place; the parity tests hold both forms to 1e-12 per pass.
 #include <cstdio>
 #include <cstring>
 
@@ -47,6 +49,9 @@ struct ShapeConst {
 };
 __constant__ ShapeConst c_shape;
 
+static void set_tables_ff(const double (&axN)[3], const double (&axD)[2], const double (&hxD)[3]);
+static bool set_tolerances_ff(double polar, double radial);
+
 void set_shape_tables()
 {
   ShapeConst s;
@@ -64,6 +69,7 @@ void set_shape_tables()
   s.hxD[2] = (2.0 - sqrt(3.0)) / 12.0;
   tet10_tables(s.t10N, s.t10D);
   cudaMemcpyToSymbol(c_shape, &s, sizeof s);
+  set_tables_ff(s.axN, s.axD, s.hxD);
 }
 
 // Limits of the element pass's bounded loops: Jacobi passes of the polar decomposition (a
@@ -89,7 +95,8 @@ __constant__ double c_returnTol = kRadialReturnPrecision;
 int set_stop_tolerances(double polar, double radial)
 {
   return cudaMemcpyToSymbol(c_polarTol, &polar, sizeof polar) == cudaSuccess &&
-                 cudaMemcpyToSymbol(c_returnTol, &radial, sizeof radial) == cudaSuccess
+                 cudaMemcpyToSymbol(c_returnTol, &radial, sizeof radial) == cudaSuccess &&
+                 set_tolerances_ff(polar, radial)
              ? 0
              : DNL_ERR_CUDA;
 }
@@ -393,42 +400,21 @@ __device__ __forceinline__ void jacobi_rotate(int k, double &f00, double &f11, d
   }
 }
 
-// ----------------------------------------------------------------------------- element kernel
-// One Gauss point of one element: lane `pt` of the NIP adjacent lanes that hold element e.  All
-// lanes of a warp must call it (the pressure average and the force sum are warp-collective);
-// lanes with valid == false compute on a clamped element and store nothing.  `red` is this
-// element's NIP x NEN*DIM slice of shared memory; `m` and `tm` are the element's material and
-// time/status record (one per mesh, or per instance in a batch).
-// GENERAL: the material may carry any hardening law (otherwise the power law, compiled alone).
-template <int ET, bool TAPE = false, bool GENERAL = false>
-__device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, DevTime *tm, int e,
-                                        int pt, bool valid, int lane, double *red)
+// J = sum_k dN/dxi (x) x_k and G_u = sum_k dN/dxi (x) du_k (Current field); axisymmetric: the radius
+// sum N_k x_k and sum N_k du_k,r.  Warp-collective where the element's lanes exchange edge differences.
+template <int ET>
+__device__ __forceinline__ void kinematics_f64(const ElemArgs &a, int e, int pt, const int (&node)[Elem<ET>::NEN],
+                                               double *red, double (&J)[Elem<ET>::DIM][Elem<ET>::DIM],
+                                               double (&GU)[Elem<ET>::DIM][Elem<ET>::DIM], double &Rad, double &vR)
 {
-  using T = Elem<ET>;
-  using L = IpLayout<ET>;
   using SH = Shape<ET>;
-  using TL = TapeLayout<ET>;
-  constexpr int NIP = T::NIP, NEN = T::NEN, DIM = T::DIM, NS = T::NS;
-  constexpr bool AXI = ET == DNL_ELQUA4NAX;  // radius, hoop strain and hoop force
-  constexpr bool TWO_D = DIM == 2;           // the 2 + 1 block structure of F, C, R, S
-  const long nIP = (long)a.E * NIP;
-  const long ipx = (long)e * NIP + pt;
-  auto tape = [&](int slot, double v) {
-    if (TAPE && valid) a.tape[(long)slot * nIP + ipx] = v;
-  };
-
-  int node[NEN];
-#pragma unroll
-  for (int k = 0; k < NEN; k++) node[k] = __ldg(a.conn + (long)k * a.E + e);
-
-  // ---- kinematics: J = sum_k dN/dxi (x) x_k and G_u = sum_k dN/dxi (x) du_k (Current field)
-  double J[DIM][DIM], GU[DIM][DIM];
+  constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
+  constexpr bool AXI = ET == DNL_ELQUA4NAX;
 #pragma unroll
   for (int r = 0; r < DIM; r++)
 #pragma unroll
     for (int c = 0; c < DIM; c++) J[r][c] = GU[r][c] = 0.;
-  double Rad = 0.;  // axisymmetric radius at the Gauss point, sum N_k x_k
-  double vR = 0.;   // axisymmetric sum N_k du_k,r
+  Rad = vR = 0.;
   constexpr bool EDGES = ET == DNL_ELHEX8N3D || ET == DNL_ELQUA4NAX || ET == DNL_ELQUA4N2D;
   if constexpr (EDGES) {
     // the element's edge differences of x and du, a few per lane, exchanged through its shared
@@ -490,15 +476,19 @@ __device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, De
       }
     }
   }
-  double detJ, Ji[DIM][DIM];
-  if (TWO_D) {
+}
+
+// J^-1 by cofactors and one reciprocal
+template <int DIM>
+__device__ __forceinline__ void inverse_f64(const double (&J)[DIM][DIM], double &detJ, double (&Ji)[DIM][DIM])
+{
+  if constexpr (DIM == 2) {
     detJ = fma(J[0][0], J[1][1], -J[0][1] * J[1][0]);
     const double r = nr_rcp(detJ);  // the IEEE reciprocal but in rare hard cases (within an ulp)
     Ji[0][0] = J[1][1] * r;
     Ji[0][1] = -J[0][1] * r;
     Ji[1][0] = -J[1][0] * r;
     Ji[1][1] = J[0][0] * r;
-    if (detJ < 0. && valid) record_error(tm, DNL_ERR_NEG_DETJ, a.eBase + e);
   } else {
     const double c00 = fma(J[1][1], J[2][2], -J[1][2] * J[2][1]);
     const double c01 = fma(J[1][2], J[2][0], -J[1][0] * J[2][2]);
@@ -514,20 +504,18 @@ __device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, De
     Ji[0][2] = fma(J[0][1], J[1][2], -J[0][2] * J[1][1]) * r;
     Ji[1][2] = fma(J[0][2], J[1][0], -J[0][0] * J[1][2]) * r;
     Ji[2][2] = fma(J[0][0], J[1][1], -J[0][1] * J[1][0]) * r;
-    if (detJ == 0. && valid) record_error(tm, DNL_ERR_SINGULAR, a.eBase + e);
   }
-  if (TAPE) {
-#pragma unroll
-    for (int l = 0; l < DIM; l++)
-#pragma unroll
-      for (int c = 0; c < DIM; c++) tape(TL::JI + l * DIM + c, Ji[l][c]);
-    tape(TL::DETJ, detJ);
-    tape(TL::RAD, Rad);
-  }
+}
 
-  // ---- F = I + sum_k du_k (x) dN_k = I + G_u J^-1 (no per-node physical gradients); the
-  // diagonal's sums are added to 1 last
-  double F[3][3] = {{1., 0., 0.}, {0., 1., 0.}, {0., 0., 1.}};
+// F = I + sum_k du_k (x) dN_k = I + G_u J^-1 (no per-node physical gradients); the diagonal's sums
+// are added to 1 last
+template <int DIM>
+__device__ __forceinline__ void gradient_f64(const double (&GU)[DIM][DIM], const double (&Ji)[DIM][DIM], double (&F)[3][3])
+{
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) F[i][j] = i == j ? 1. : 0.;
 #pragma unroll
   for (int r = 0; r < DIM; r++)
 #pragma unroll
@@ -537,24 +525,12 @@ __device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, De
       for (int l = 0; l < DIM; l++) s = fma(GU[r][l], Ji[l][c], s);
       F[r][c] = r == c ? RADD(1.0, s) : s;
     }
-  // hoop stretch u_r / R by a reciprocal and one residual correction (quot)
-  double vRR = 0.;
-  if (AXI) {
-    vRR = quot(vR, Rad, nr_rcp(Rad));
-    F[2][2] = RADD(F[2][2], vRR);
-  }
-  if (TAPE) {
-#pragma unroll
-    for (int k = 0; k < 9; k++) tape(TL::F + k, F[k / 3][k % 3]);
-#pragma unroll
-    for (int r = 0; r < DIM; r++)
-#pragma unroll
-      for (int l = 0; l < DIM; l++) tape(TL::GU + r * DIM + l, GU[r][l]);
-    tape(TL::VRR, vRR);
-  }
+}
 
-  // ---- C = F^T F (Tensor2::Transpose then operator*), exact reference rounding
-  double f[3][3];
+// C = F^T F (Tensor2::Transpose then operator*), exact reference rounding
+template <bool TWO_D>
+__device__ __forceinline__ void cauchy_f64(const double (&F)[3][3], double (&f)[3][3])
+{
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
@@ -572,6 +548,75 @@ __device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, De
       f[i][j] = s;
       f[j][i] = s;
     }
+}
+
+// ----------------------------------------------------------------------------- element kernel
+// One Gauss point of one element: lane `pt` of the NIP adjacent lanes that hold element e.  All
+// lanes of a warp must call it (the pressure average and the force sum are warp-collective);
+// lanes with valid == false compute on a clamped element and store nothing.  `red` is this
+// element's NIP x NEN*DIM slice of shared memory; `m` and `tm` are the element's material and
+// time/status record (one per mesh, or per instance in a batch).
+// GENERAL: the material may carry any hardening law (otherwise the power law, compiled alone).
+template <int ET, bool TAPE = false, bool GENERAL = false>
+__device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, DevTime *tm, int e,
+                                        int pt, bool valid, int lane, double *red)
+{
+  using T = Elem<ET>;
+  using L = IpLayout<ET>;
+  using SH = Shape<ET>;
+  using TL = TapeLayout<ET>;
+  constexpr int NIP = T::NIP, NEN = T::NEN, DIM = T::DIM, NS = T::NS;
+  constexpr bool AXI = ET == DNL_ELQUA4NAX;  // radius, hoop strain and hoop force
+  constexpr bool TWO_D = DIM == 2;           // the 2 + 1 block structure of F, C, R, S
+  const long nIP = (long)a.E * NIP;
+  const long ipx = (long)e * NIP + pt;
+  auto tape = [&](int slot, double v) {
+    if (TAPE && valid) a.tape[(long)slot * nIP + ipx] = v;
+  };
+
+  int node[NEN];
+#pragma unroll
+  for (int k = 0; k < NEN; k++) node[k] = __ldg(a.conn + (long)k * a.E + e);
+
+  // ---- kinematics
+  double J[DIM][DIM], GU[DIM][DIM], Rad, vR;
+  kinematics_f64<ET>(a, e, pt, node, red, J, GU, Rad, vR);
+  double detJ, Ji[DIM][DIM];
+  inverse_f64(J, detJ, Ji);
+  if (TWO_D) {
+    if (detJ < 0. && valid) record_error(tm, DNL_ERR_NEG_DETJ, a.eBase + e);
+  } else {
+    if (detJ == 0. && valid) record_error(tm, DNL_ERR_SINGULAR, a.eBase + e);
+  }
+  if (TAPE) {
+#pragma unroll
+    for (int l = 0; l < DIM; l++)
+#pragma unroll
+      for (int c = 0; c < DIM; c++) tape(TL::JI + l * DIM + c, Ji[l][c]);
+    tape(TL::DETJ, detJ);
+    tape(TL::RAD, Rad);
+  }
+
+  double F[3][3];
+  gradient_f64(GU, Ji, F);
+  // hoop stretch u_r / R by a reciprocal and one residual correction (quot)
+  double vRR = 0.;
+  if (AXI) {
+    vRR = quot(vR, Rad, nr_rcp(Rad));
+    F[2][2] = RADD(F[2][2], vRR);
+  }
+  if (TAPE) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) tape(TL::F + k, F[k / 3][k % 3]);
+#pragma unroll
+    for (int r = 0; r < DIM; r++)
+#pragma unroll
+      for (int l = 0; l < DIM; l++) tape(TL::GU + r * DIM + l, GU[r][l]);
+    tape(TL::VRR, vRR);
+  }
+
+  double f[3][3];
+  cauchy_f64<TWO_D>(F, f);
 
   // ---- Jacobi eigen-iteration (at most 29 rotations, c_caps[0]; Tensor2.C:1169)
   double rot[3][3] = {{1., 0., 0.}, {0., 1., 0.}, {0., 0., 1.}};
@@ -1067,12 +1112,55 @@ __device__ __forceinline__ void elem_ip(const ElemArgs &a, const Material &m, De
   }
 }
 
+#include "dnl_elem_ff.cuh"
+// doubles of shared memory per element: edge differences and the exchange of the points' products
+// (quads, hexahedron), else the points' rows of nodal forces
+__host__ __device__ constexpr int etype_slots(int et)
+{
+  return et == DNL_ELHEX8N3D ? 72 : (etype_quad(et) ? 24 : etype_nip(et) * etype_nen(et) * etype_dim(et));
+}
+
+// the FP64 pass as a call: the pair pass's registers are not held over it
+template <int ET, bool TAPE, bool GENERAL>
+__device__ __noinline__ void elem_f64(const ElemArgs &a, const Material &m, DevTime *tm, int e, int pt, bool valid,
+                                      int lane, double *red)
+{
+  elem_ip<ET, TAPE, GENERAL>(a, m, tm, e, pt, valid, lane, red);
+}
+
+// One Gauss point: in pairs, and the FP64 pass for the elements of the warp that need it.
 template <int ET, bool TAPE = false, bool GENERAL = false>
-__global__ void __launch_bounds__(128) k_elem(ElemArgs a)
+__device__ __forceinline__ void elem_point(const ElemArgs &a, const Material &m, DevTime *tm, int e, int pt,
+                                           bool valid, int lane, double *red, float2 *hold)
+{
+  if constexpr (etype_fast(ET)) {
+    const bool slow = elem_fast<ET, TAPE, GENERAL>(a, m, tm, e, pt, valid, lane, red, hold);
+    if (__any_sync(0xffffffffu, slow && valid)) {
+      __syncwarp();
+      elem_f64<ET, TAPE, GENERAL>(a, m, tm, e, pt, slow && valid, lane, red);
+    }
+  } else {
+    elem_ip<ET, TAPE, GENERAL>(a, m, tm, e, pt, valid, lane, red);
+  }
+}
+
+// Blocks per SM the register allocation aims at.  The pair pass of the 3D elements has instruction
+// level parallelism but long straight-line code, and waits for its instructions more than for anything
+// else: more warps hide that until the spills cost more (505,600 hexahedra: 1.93 ms unbounded at
+// 168 registers, 1.74 at 128, 1.77 at 96; 207,872 one-point hexahedra 272 us at 232, 182 at 128).  The quads
+// and the tetrahedron, and the instances with a record or general hardening, are faster unbounded.
+constexpr int elem_min_blocks(int et, bool tape, bool general)
+{
+  return !tape && !general && (et == DNL_ELHEX8N3D || et == DNL_ELHEX8N3D_1PT) ? 4 : 1;
+}
+
+template <int ET, bool TAPE = false, bool GENERAL = false>
+__global__ void __launch_bounds__(128, elem_min_blocks(ET, TAPE, GENERAL)) k_elem(const __grid_constant__ ElemArgs a)
 {
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int EPW = 32 / NIP;  // elements per warp
-  __shared__ double red[128 / 32][EPW][NIP * NEN * DIM];
+  __shared__ double red[128 / 32][EPW][etype_slots(ET)];
+  __shared__ float2 hold[128 / 32][etype_fast(ET) ? hold_slots<ET>() * HOLD : 1];
   if (a.gate && (a.tm->done | a.tm->status)) return;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   if ((gtid & ~31) / NIP >= a.E) return;
@@ -1081,23 +1169,24 @@ __global__ void __launch_bounds__(128) k_elem(ElemArgs a)
   const int lane = threadIdx.x & 31;
   const int e = valid ? eRaw : a.E - 1;
   if (GENERAL && a.elemMat)
-    elem_ip<ET, TAPE, true>(a, a.mats[a.elemMat[e]], a.tm, e, gtid % NIP, valid, lane,
-                            red[threadIdx.x >> 5][lane / NIP]);
+    elem_point<ET, TAPE, true>(a, a.mats[a.elemMat[e]], a.tm, e, gtid % NIP, valid, lane,
+                               red[threadIdx.x >> 5][lane / NIP], hold[threadIdx.x >> 5] + lane);
   else
-    elem_ip<ET, TAPE, GENERAL>(a, a.mat, a.tm, e, gtid % NIP, valid, lane,
-                               red[threadIdx.x >> 5][lane / NIP]);
+    elem_point<ET, TAPE, GENERAL>(a, a.mat, a.tm, e, gtid % NIP, valid, lane,
+                                  red[threadIdx.x >> 5][lane / NIP], hold[threadIdx.x >> 5] + lane);
 }
 
 // Batched element pass over the union of many meshes: element e belongs to instance inst[e],
 // whose material and time record are mats[inst] and tms[inst]; instances that have finished or
 // failed keep their lanes in the warp but store nothing.
 template <int ET, int BLOCK, bool TAPE = false>
-__global__ void __launch_bounds__(BLOCK) k_elem_batch(ElemArgs a, const int *elemInst,
+__global__ void __launch_bounds__(BLOCK) k_elem_batch(const __grid_constant__ ElemArgs a, const int *elemInst,
                                                       const Material *mats, DevTime *tms)
 {
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int EPW = 32 / NIP;
-  __shared__ double red[BLOCK / 32][EPW][NIP * NEN * DIM];
+  __shared__ double red[BLOCK / 32][EPW][etype_slots(ET)];
+  __shared__ float2 hold[BLOCK / 32][etype_fast(ET) ? hold_slots<ET>() * HOLD : 1];
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   if ((gtid & ~31) / NIP >= a.E) return;
   const int eRaw = gtid / NIP;
@@ -1106,7 +1195,8 @@ __global__ void __launch_bounds__(BLOCK) k_elem_batch(ElemArgs a, const int *ele
   DevTime *tm = tms + inst;
   const bool valid = eRaw < a.E && !(tm->done | tm->status);
   const int lane = threadIdx.x & 31;
-  elem_ip<ET, TAPE>(a, mats[inst], tm, e, gtid % NIP, valid, lane, red[threadIdx.x >> 5][lane / NIP]);
+  elem_point<ET, TAPE>(a, mats[inst], tm, e, gtid % NIP, valid, lane, red[threadIdx.x >> 5][lane / NIP],
+                       hold[threadIdx.x >> 5] + lane);
 }
 
 // ----------------------------------------------------------------------------- tangent pass
@@ -1349,11 +1439,12 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err)
 }
 
 template <int ET, int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_batch_persistent(BatchStepArgs a)
+__global__ void __launch_bounds__(BLOCK) k_batch_persistent(const __grid_constant__ BatchStepArgs a)
 {
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int EPW = 32 / NIP;
-  __shared__ double red[BLOCK / 32][EPW][NIP * NEN * DIM];
+  __shared__ double red[BLOCK / 32][EPW][etype_slots(ET)];
+  __shared__ float2 hold[BLOCK / 32][hold_slots<ET>() * HOLD];
   const int tid = blockIdx.x * BLOCK + threadIdx.x, nthreads = gridDim.x * BLOCK;
   // ---- time logic: initStep of every unfinished instance
   if (a.preFirst) {
@@ -1398,8 +1489,8 @@ __global__ void __launch_bounds__(BLOCK) k_batch_persistent(BatchStepArgs a)
       const int inst = a.elemInst[e];
       DevTime *tm = a.tms + inst;
       const bool valid = eRaw < a.ea.E && !(tm->done | tm->status);
-      elem_ip<ET>(a.ea, a.mats[inst], tm, e, (int)(gtid % NIP), valid, lane,
-                  red[threadIdx.x >> 5][lane / NIP]);
+      elem_point<ET>(a.ea, a.mats[inst], tm, e, (int)(gtid % NIP), valid, lane,
+                     red[threadIdx.x >> 5][lane / NIP], hold[threadIdx.x >> 5] + lane);
       __syncwarp();
     }
   }
@@ -1602,8 +1693,8 @@ int launch_mass(dnl_handle *h, cudaStream_t s, double *me)
 int launch_elem_batch(int etype, int block, const ElemArgs &a, const int *elemInst,
                       const Material *mats, DevTime *tms, cudaStream_t s)
 {
-  // the hexahedra's and the 10-node tetrahedron's shared-memory transpose fits 128 threads at most
-  if ((etype == DNL_ELHEX8N3D || etype == DNL_ELTET10N3D || etype == DNL_ELHEX8N3D_1PT) && block > 128)
+  // the solid elements' shared memory fits 128 threads at most
+  if (!etype_quad(etype) && block > 128)
     block = 128;
   const long threads = (long)a.E * etype_nip(etype);
   const int grid = (int)((threads + block - 1) / block);
@@ -1613,7 +1704,6 @@ int launch_elem_batch(int etype, int block, const ElemArgs &a, const int *elemIn
     else DNL_EB(DNL_ELHEX8N3D_1PT, 128);
   } else if (etype == DNL_ELTET4N3D) {
     if (block == 64) DNL_EB(DNL_ELTET4N3D, 64);
-    else if (block == 256) DNL_EB(DNL_ELTET4N3D, 256);
     else DNL_EB(DNL_ELTET4N3D, 128);
   } else if (etype == DNL_ELTET10N3D) {
     if (block == 64) DNL_EB(DNL_ELTET10N3D, 64);

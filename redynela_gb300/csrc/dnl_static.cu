@@ -52,6 +52,7 @@ int static_setup(StaticPtrs **out)
     dnl::DevTime *tm = nullptr;
     if (cudaGetSymbolAddress((void **)&fe, g_static_fe) != cudaSuccess) return DNL_ERR_CUDA;
     if (cudaGetSymbolAddress((void **)&tm, g_static_tm) != cudaSuccess) return DNL_ERR_CUDA;
+    dnl::set_shape_tables();  // the element tables: no handle need exist
     p.fe = fe;
     p.tm = tm;
     p.ready = true;
