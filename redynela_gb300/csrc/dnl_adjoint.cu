@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "dnl_common.cuh"
+#include "dnl_node.cuh"
 
 namespace dnl {
 
@@ -92,20 +93,8 @@ void adj_drop_graphs(AdjState *A)
   A->graphs.clear();
 }
 
-// the time record between scheduled steps: phase 0 initStep with the scheduled step, 1 updateTime,
-// 2 both (updateTime of one step then initStep of the next: one launch between two steps)
-__global__ void k_adj_dt(DevTime *tm, const double *dts, int phase)
-{
-  if (tm->status) return;
-  if (phase != 0)  // updateTime
-    tm->currentTime = __dadd_rn(tm->currentTime, tm->timeStep);
-  if (phase != 1) {  // initStep with the scheduled step
-    const double dt = dts[tm->increment];
-    tm->timeStep = dt;
-    tm->nextTime = __dadd_rn(tm->currentTime, dt);
-    tm->increment++;
-  }
-}
+// opens a sequence of scheduled steps (sched_update); the nodal update's last block runs the others
+__global__ void k_adj_dt(DevTime *tm, const double *dts) { sched_update(tm, dts, 0); }
 
 // a step's record: the coordinates (3N), the Current delta_disp (3N) and the integration-point
 // state (n doubles) copied into rec one after another, in one launch
@@ -357,18 +346,18 @@ int adj_alloc(dnl_handle *h, AdjState *A, int nsteps, int stride)
 // the coordinates, the Current delta_disp and the integration-point state the element pass reads
 // are copied there first
 // `first`: the step opens with initStep; `last`: it ends with updateTime; between two steps of a
-// sequence one launch does both (the same operations in the same order)
+// sequence the nodal update's last block does both (the same operations in the same order)
 int adj_primal_step(dnl_handle *h, const double *dtsDev, double *rec, double *tapeOut = nullptr,
                     bool first = true, bool last = true)
 {
   cudaStream_t s = h->stream;
   const size_t N = h->N, nIP = ip_total(h);  // one allocation holds every group's state
   if (first) {
-    k_adj_dt<<<1, 1, 0, s>>>(h->tm, dtsDev, 0);
+    k_adj_dt<<<1, 1, 0, s>>>(h->tm, dtsDev);
     launch_counter()++;
   }
   int r;
-  if ((r = enqueue_bc_current(h))) return r;
+  if ((r = enqueue_bc_current(h, first))) return r;
   if (rec) {
     const long total = 6 * (long)N + (long)ip_ncomp(h->etype) * nIP;
     k_adj_record<<<(unsigned)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096), 256, 0, s>>>(
@@ -377,10 +366,12 @@ int adj_primal_step(dnl_handle *h, const double *dtsDev, double *rec, double *ta
   }
   // with tapeOut: the same pass (bit for bit) also writing its per-point record there
   if ((r = tapeOut ? launch_elem_tape(h, s, tapeOut) : launch_elem(h, s, 1))) return r;
-  if ((r = enqueue_node(h))) return r;
+  StepTail tail;
+  memset(&tail, 0, sizeof tail);
+  tail.sched = last ? 1 : 2;
+  tail.dts = dtsDev;
+  if ((r = enqueue_node(h, tail))) return r;
   h->cur = 1 - h->cur;
-  k_adj_dt<<<1, 1, 0, s>>>(h->tm, dtsDev, last ? 1 : 2);
-  launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
 

@@ -149,26 +149,35 @@ int enqueue_batch_step_persistent(dnl_batch *b, long long incAfter, bool first, 
   return r;
 }
 
-int enqueue_batch_step(dnl_batch *b, long long incAfter, bool last)
+int enqueue_batch_step(dnl_batch *b, long long incAfter, bool first, bool last)
 {
   dnl_handle *h = b->h;
   int r;
-  if ((r = launch_bc_batch(h, b->tms, b->nodeInst))) return r;
+  if ((r = launch_bc_batch(h, b->tms, b->nodeInst, first))) return r;
   ElemArgs a = elem_args_of(h);
   prof_begin(h, h->stream);
   r = launch_elem_batch(h->etype, b->block, a, b->elemInst, b->mats, b->tms, h->stream);
   prof_end(h, DNL_PROF_ELEM, h->stream);
   if (r) return r;
-  if ((r = launch_node_batch(h, b->nodeInst, b->prm, b->tms))) return r;
+  // the time logic of every instance in the last block of the step's last kernel
+  StepTail none, tail;
+  memset(&none, 0, sizeof none);
+  memset(&tail, 0, sizeof tail);
+  tail.mode = last ? BT_POST : (BT_POST | BT_PRE);
+  tail.count = b->count;
+  tail.tms = b->tms;
+  tail.prm = b->prm;
+  const bool due = incAfter % b->freq == 0;
+  if ((r = launch_node_batch(h, b->nodeInst, b->prm, b->tms, due ? none : tail))) return r;
   h->cur = 1 - h->cur;
-  if (incAfter % b->freq == 0) {
+  if (due) {
     ElemArgs c = elem_args_of(h);
     prof_begin(h, h->stream);
-    r = launch_courant_batch(h->etype, c, b->elemInst, b->tms, h->stream);
+    r = launch_courant_batch(h->etype, c, b->elemInst, b->tms, h->stream, tail);
     prof_end(h, DNL_PROF_COURANT, h->stream);
     if (r) return r;
   }
-  return launch_dt_batch(h, b->tms, b->prm, b->count, last ? BT_POST : (BT_POST | BT_PRE));
+  return 0;
 }
 
 // evp^n of every integration point with its instance's n (the cached yield term), after a state
@@ -193,7 +202,7 @@ int enqueue_steps(dnl_batch *b, long long inc0, int nsteps)
   }
   if ((r = launch_dt_batch(h, b->tms, b->prm, b->count, BT_PRE))) return r;
   for (int s = 0; s < nsteps; s++)
-    if ((r = enqueue_batch_step(b, inc0 + s + 1, s == nsteps - 1))) return r;
+    if ((r = enqueue_batch_step(b, inc0 + s + 1, s == 0, s == nsteps - 1))) return r;
   return 0;
 }
 
@@ -435,7 +444,9 @@ int dnl_batch_prologue(dnl_batch *b)
   // computeInternalForces with the initial (zero) Current field, then computeTimeStep(True)
   ElemArgs a = elem_args_of(h);
   if ((r = launch_elem_batch(h->etype, b->block, a, b->elemInst, b->mats, b->tms, h->stream))) return r;
-  if ((r = launch_courant_batch(h->etype, a, b->elemInst, b->tms, h->stream))) return r;
+  StepTail none;
+  memset(&none, 0, sizeof none);
+  if ((r = launch_courant_batch(h->etype, a, b->elemInst, b->tms, h->stream, none))) return r;
   if ((r = launch_dt_batch(h, b->tms, b->prm, b->count, BT_FORCE))) return r;
   std::vector<DevTime> t;
   if ((r = read_tms(b, t))) return r;

@@ -195,7 +195,7 @@ struct DevTime {
   int badElem;
   int pulseDone;                     // Pulse: power iteration converged
   int pulseIter;                     // Pulse: iterations of the running call
-  int pad;
+  unsigned arrived;                  // blocks of the running kernel past their work (step_tail); 0 between
 };
 
 // ------------------------------------------------------------------------ kernel arguments
@@ -348,6 +348,19 @@ struct GatherArgs {
   double *fint;           // [N*DIM], Id*dim+j
 };
 
+// The time logic that closes a step, run by the last block of the step's last kernel instead of a
+// launch of its own (dnl_node.cuh): mode bits DT_* (0: none), or with dts the scheduled steps'
+// phases (sched: 1 updateTime, 2 updateTime and the next initStep).  In a batch the records are tms,
+// their constants prm.
+struct StepTail {
+  int mode, freq, method, sched;
+  double safetyOmega, Cs;
+  const double *dts;
+  int count;               // batched: instances
+  DevTime *tms;
+  const struct InstParams *prm;
+};
+
 struct NodeArgs {
   int N, EN;
   const int *start, *entry;
@@ -361,6 +374,7 @@ struct NodeArgs {
   double *fint;           // optional [N*DIM] copy of the assembled forces
   DevTime *tm;
   double alphaM, beta, gamma;
+  StepTail tail;
 };
 
 // per-instance constants of a batch
@@ -585,12 +599,13 @@ int sens_schedule(dnl_handle *h, const double **dts, int *n);
 int sens_outputs(dnl_handle *h, double *coords, double *dcoords);
 void sens_free(dnl_handle *h);
 // primal per-step launches (dnl_host.cu) used by the sensitivity run
-int enqueue_bc_current(dnl_handle *h);
-int enqueue_node(dnl_handle *h);
+// firstOfCall: the Current fields may have been changed since the last step (see launch_bc_current)
+int enqueue_bc_current(dnl_handle *h, bool firstOfCall);
+int enqueue_node(dnl_handle *h, const StepTail &tail);
 int read_time_state(dnl_handle *h, DevTime *t);
 int restart_time(dnl_handle *h, double t);
 int launch_mass(dnl_handle *h, cudaStream_t s, double *me);
-int launch_courant(dnl_handle *h, cudaStream_t s);
+int launch_courant(dnl_handle *h, cudaStream_t s, const StepTail &tail);
 int launch_pulse(dnl_handle *h, cudaStream_t s);
 void set_shape_tables();
 // loop limits of the element pass (Jacobi passes, Newton iterations; device constants of the
@@ -605,15 +620,16 @@ int launch_elem_batch(int etype, int block, const ElemArgs &a, const int *elemIn
 int launch_mass_batch(int etype, const ElemArgs &a, double *me, const int *elemInst,
                       const Material *mats, cudaStream_t s);
 int launch_courant_batch(int etype, const ElemArgs &a, const int *elemInst, DevTime *tms,
-                         cudaStream_t s);
+                         cudaStream_t s, const StepTail &tail);
 // one batched step as a persistent cooperative launch (ElQua4nAx); grid from the occupancy
 int launch_batch_persistent(int etype, int block, const BatchStepArgs &a, cudaStream_t s);
 ElemArgs elem_args_of(dnl_handle *h);
 // the element pass's arguments for element group gi (-1: the first group, as elem_args_of)
 ElemArgs group_args_of(dnl_handle *h, int gi);
-int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm, DevTime *tms);
+int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm, DevTime *tms,
+                      const StepTail &tail);
 int launch_dt_batch(dnl_handle *h, DevTime *tms, const InstParams *prm, int count, int mode);
-int launch_bc_batch(dnl_handle *h, DevTime *tms, const int *nodeInst);
+int launch_bc_batch(dnl_handle *h, DevTime *tms, const int *nodeInst, bool firstOfCall);
 int launch_gather_mass(dnl_handle *h, const double *me);
 // launches on caller-built arguments (no handle)
 int launch_elem_raw(int etype, const ElemArgs &a, cudaStream_t s);

@@ -1349,7 +1349,7 @@ __device__ __forceinline__ double elem_length(const ElemArgs &a, int e)
 // their bits).  A non-positive or NaN length is an error: the reference would turn it into a
 // negative or NaN time step.
 template <int KIND>
-__global__ void __launch_bounds__(256) k_courant(ElemArgs a)
+__global__ void __launch_bounds__(256) k_courant(ElemArgs a, StepTail tail)
 {
   if (a.tm->done | a.tm->status) return;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1373,12 +1373,13 @@ __global__ void __launch_bounds__(256) k_courant(ElemArgs a)
     for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = fmin(b, wmin[w]);
     atomicMin(&a.tm->lenMinBits, (unsigned long long)__double_as_longlong(b));
   }
+  step_tail(tail, a.tm);
 }
 
 // Batched Courant lengths: each element folds its length into its instance's minimum; a warp whose
 // lanes all belong to one instance reduces first and issues one atomic.
 template <int KIND>
-__global__ void __launch_bounds__(256) k_courant_batch(ElemArgs a, const int *elemInst, DevTime *tms)
+__global__ void __launch_bounds__(256) k_courant_batch(ElemArgs a, const int *elemInst, DevTime *tms, StepTail tail)
 {
   const int eRaw = blockIdx.x * blockDim.x + threadIdx.x;
   if ((eRaw & ~31) >= a.E) return;
@@ -1402,6 +1403,7 @@ __global__ void __launch_bounds__(256) k_courant_batch(ElemArgs a, const int *el
   } else if (len < 1e300) {
     atomicMin(&tm->lenMinBits, (unsigned long long)__double_as_longlong(len));
   }
+  step_tail(tail, tms);
 }
 
 // ----------------------------------------------------------------------------- persistent batch step
@@ -1748,15 +1750,15 @@ int launch_mass_batch(int etype, const ElemArgs &a, double *me, const int *elemI
 }
 
 int launch_courant_batch(int etype, const ElemArgs &a, const int *elemInst, DevTime *tms,
-                         cudaStream_t s)
+                         cudaStream_t s, const StepTail &tail)
 {
   const int kind = etype_length_kind(etype), grid = (a.E + 255) / 256;
   if (kind == 0)
-    k_courant_batch<0><<<grid, 256, 0, s>>>(a, elemInst, tms);
+    k_courant_batch<0><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
   else if (kind == 1)
-    k_courant_batch<1><<<grid, 256, 0, s>>>(a, elemInst, tms);
+    k_courant_batch<1><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
   else
-    k_courant_batch<2><<<grid, 256, 0, s>>>(a, elemInst, tms);
+    k_courant_batch<2><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
@@ -1764,20 +1766,23 @@ int launch_courant_batch(int etype, const ElemArgs &a, const int *elemInst, DevT
 ElemArgs elem_args_of(dnl_handle *h) { return elem_args(h); }
 ElemArgs group_args_of(dnl_handle *h, int gi) { return gi < 0 ? elem_args(h) : group_args(h, h->extra[gi]); }
 
-int launch_courant(dnl_handle *h, cudaStream_t s)
+int launch_courant(dnl_handle *h, cudaStream_t s, const StepTail &tail)
 {
+  StepTail none;
+  memset(&none, 0, sizeof none);
   prof_begin(h, s);
   // every element group's lengths into the one minimum (its kernels reduce into the time record)
   for (int gi = -1; gi < h->nextra; gi++) {
     const ElemArgs a = gi < 0 ? elem_args(h) : group_args(h, h->extra[gi]);
     const int et = gi < 0 ? h->etype : h->extra[gi].etype;
     const int kind = etype_length_kind(et), grid = (a.E + 255) / 256;
+    const StepTail &t = gi == h->nextra - 1 ? tail : none;  // the last group's kernel ends the step
     if (kind == 0)
-      k_courant<0><<<grid, 256, 0, s>>>(a);
+      k_courant<0><<<grid, 256, 0, s>>>(a, t);
     else if (kind == 1)
-      k_courant<1><<<grid, 256, 0, s>>>(a);
+      k_courant<1><<<grid, 256, 0, s>>>(a, t);
     else
-      k_courant<2><<<grid, 256, 0, s>>>(a);
+      k_courant<2><<<grid, 256, 0, s>>>(a, t);
     launch_counter()++;
   }
   prof_end(h, DNL_PROF_COURANT, s);

@@ -70,10 +70,10 @@ template <int DIM>
 __global__ void __launch_bounds__(256) k_node(NodeArgs g)
 {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= g.N) return;
   DevTime *tm = g.tm;
-  if (tm->done | tm->status) return;
-  node_update<DIM>(g, n, tm->timeStep, g.alphaM, g.beta, g.gamma);
+  if (tm->done | tm->status) return;  // set by earlier kernels or by this one's last block: all blocks alike
+  if (n < g.N) node_update<DIM>(g, n, tm->timeStep, g.alphaM, g.beta, g.gamma);
+  step_tail(g.tail, tm);
 }
 
 // batched: node n belongs to instance nodeInst[n] with its own time record and constants
@@ -82,11 +82,12 @@ __global__ void __launch_bounds__(256) k_node_batch(NodeArgs g, const int *nodeI
                                                     const InstParams *prm, DevTime *tms)
 {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= g.N) return;
-  const int i = nodeInst[n];
-  const DevTime *tm = tms + i;
-  if (tm->done | tm->status) return;
-  node_update<DIM>(g, n, tm->timeStep, prm[i].alphaM, prm[i].beta, prm[i].gamma);
+  if (n < g.N) {
+    const int i = nodeInst[n];
+    const DevTime *tm = tms + i;
+    if (!(tm->done | tm->status)) node_update<DIM>(g, n, tm->timeStep, prm[i].alphaM, prm[i].beta, prm[i].gamma);
+  }
+  step_tail(g.tail, tms);
 }
 
 // Current-field writes of the constant boundary conditions before the element pass; in a batch
@@ -162,15 +163,9 @@ __global__ void k_bc_current_va(int nb, const int *nodes, const int *code, const
 }
 
 // ----------------------------------------------------------------------------- time step
-struct DtArgs {
-  DevTime *tm;
-  int mode, freq, method;
-  double safetyOmega, Cs;
-};
-
-__global__ void k_dt(DtArgs a)
+__global__ void k_dt(DevTime *tm, StepTail a)
 {
-  dt_update(a.tm, a.mode, a.freq, a.method, a.safetyOmega, a.Cs);
+  dt_update(tm, a.mode, a.freq, a.method, a.safetyOmega, a.Cs);
 }
 
 __global__ void k_dt_batch(DevTime *tms, const InstParams *prm, int count, int mode)
@@ -345,9 +340,23 @@ int launch_gather(dnl_handle *h)
   return check_launch();
 }
 
-int launch_node(dnl_handle *h, bool keepFint)
+// the time logic of the handle's steps for a kernel's last block
+StepTail step_tail_args(dnl_handle *h, int mode)
+{
+  StepTail t;
+  memset(&t, 0, sizeof t);
+  t.mode = mode;
+  t.freq = h->freq;
+  t.method = h->method;
+  t.safetyOmega = h->safetyOmega;
+  t.Cs = h->elemCs ? 1.0 : h->mat.Cs;  // several materials: k_courant reduced len / Cs per element
+  return t;
+}
+
+int launch_node(dnl_handle *h, bool keepFint, const StepTail &tail)
 {
   NodeArgs g;
+  g.tail = tail;
   g.N = h->N;
   g.EN = (int)h->EN;
   g.start = h->n2eStart;
@@ -378,23 +387,19 @@ int launch_node(dnl_handle *h, bool keepFint)
 
 int launch_dt(dnl_handle *h, int mode)
 {
-  DtArgs a;
-  a.tm = h->tm;
-  a.mode = mode;
-  a.freq = h->freq;
-  a.method = h->method;
-  a.safetyOmega = h->safetyOmega;
-  a.Cs = h->elemCs ? 1.0 : h->mat.Cs;  // several materials: k_courant reduced len / Cs per element
   prof_begin(h, h->stream);
-  k_dt<<<1, 1, 0, h->stream>>>(a);
+  k_dt<<<1, 1, 0, h->stream>>>(h->tm, step_tail_args(h, mode));
   prof_end(h, DNL_PROF_OTHER, h->stream);
   launch_counter()++;
   return check_launch();
 }
 
-int launch_bc_current(dnl_handle *h)
+// firstOfCall: between the steps of one call nothing but the nodal update writes the nodal fields,
+// and it leaves restrained components at zero itself; only imposed speeds (delta_disp follows the
+// step size) need their writes before every step.
+int launch_bc_current(dnl_handle *h, bool firstOfCall)
 {
-  if (!h->nbcNodes) return 0;
+  if (!h->nbcNodes || (!firstOfCall && !h->hasSpeedBC)) return 0;
   prof_begin(h, h->stream);
   k_bc_current<<<(h->nbcNodes + 127) / 128, 128, 0, h->stream>>>(h->nbcNodes, h->bcNodeList, h->bcCode,
                                                                   h->bcSpeed, h->bank[h->cur], h->tm,
@@ -405,10 +410,25 @@ int launch_bc_current(dnl_handle *h)
 }
 
 // critical-time-step computation that precedes a DT_FORCE or a due DT_POST
-int launch_time_step_source(dnl_handle *h)
+int launch_time_step_source(dnl_handle *h, const StepTail &tail)
 {
-  if (h->method == DNL_COURANT) return launch_courant(h, h->stream);
+  if (h->method == DNL_COURANT) return launch_courant(h, h->stream, tail);
   return launch_pulse(h, h->stream);
+}
+
+// what closes a step after its nodal update: the critical time step when due (Courant's kernel
+// runs the time logic in its last block, Pulse's call is followed by a launch of it), else nothing --
+// the nodal update's last block has run it (node_tail)
+StepTail node_tail(dnl_handle *h, long long incAfter, int mode)
+{
+  return step_tail_args(h, incAfter % h->freq == 0 ? 0 : mode);
+}
+int launch_step_end(dnl_handle *h, long long incAfter, int mode)
+{
+  if (incAfter % h->freq != 0) return 0;
+  int r;
+  if ((r = launch_time_step_source(h, step_tail_args(h, mode)))) return r;
+  return h->method == DNL_COURANT ? 0 : launch_dt(h, mode);
 }
 
 int read_time(dnl_handle *h, DevTime *out)
@@ -419,28 +439,26 @@ int read_time(dnl_handle *h, DevTime *out)
 }
 
 
-// one explicit step's launches; post = complete this step's time update afterwards
-int enqueue_step(dnl_handle *h, long long incAfter, bool last)
+// one explicit step's launches, the first and the last of a call marked
+int enqueue_step(dnl_handle *h, long long incAfter, bool first, bool last)
 {
+  const int mode = last ? DT_POST : (DT_POST | DT_PRE);
   int r;
-  if (h->hasSpeedBC || h->nbcNodes) {
-    if ((r = launch_bc_current(h))) return r;
-  }
+  if ((r = launch_bc_current(h, first))) return r;
   if ((r = launch_elem(h, h->stream, 1))) return r;
-  if ((r = launch_node(h, true))) return r;
+  if ((r = launch_node(h, true, node_tail(h, incAfter, mode)))) return r;
   h->cur = 1 - h->cur;  // endStep: Node::transfertNodalField
-  if (incAfter % h->freq == 0) {
-    if ((r = launch_time_step_source(h))) return r;
-  }
-  return launch_dt(h, last ? DT_POST : (DT_POST | DT_PRE));
+  return launch_step_end(h, incAfter, mode);
 }
 
 }  // namespace
 
 namespace dnl {
-int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm, DevTime *tms)
+int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm, DevTime *tms,
+                      const StepTail &tail)
 {
   NodeArgs g;
+  g.tail = tail;
   g.N = h->N;
   g.EN = (int)h->EN;
   g.start = h->n2eStart;
@@ -476,9 +494,9 @@ int launch_dt_batch(dnl_handle *h, DevTime *tms, const InstParams *prm, int coun
   return check_launch();
 }
 
-int launch_bc_batch(dnl_handle *h, DevTime *tms, const int *nodeInst)
+int launch_bc_batch(dnl_handle *h, DevTime *tms, const int *nodeInst, bool firstOfCall)
 {
-  if (!h->nbcNodes) return 0;
+  if (!h->nbcNodes || (!firstOfCall && !h->hasSpeedBC)) return 0;
   prof_begin(h, h->stream);
   k_bc_current<<<(h->nbcNodes + 127) / 128, 128, 0, h->stream>>>(h->nbcNodes, h->bcNodeList, h->bcCode,
                                                                   h->bcSpeed, h->bank[h->cur], tms,
@@ -507,7 +525,7 @@ int restart_time(dnl_handle *h, double t)
   k_set_time<<<1, 1, 0, h->stream>>>(h->tm, t);
   launch_counter()++;
   int r;
-  if ((r = launch_time_step_source(h))) return r;
+  if ((r = launch_time_step_source(h, step_tail_args(h, 0)))) return r;
   if ((r = launch_dt(h, DT_FORCE))) return r;
   DevTime tt;
   if ((r = read_time(h, &tt))) return r;
@@ -515,8 +533,8 @@ int restart_time(dnl_handle *h, double t)
 }
 
 // the primal per-step launches, for the sensitivity run (dnl_sens.cu)
-int enqueue_bc_current(dnl_handle *h) { return (h->hasSpeedBC || h->nbcNodes) ? launch_bc_current(h) : 0; }
-int enqueue_node(dnl_handle *h) { return launch_node(h, true); }
+int enqueue_bc_current(dnl_handle *h, bool firstOfCall) { return launch_bc_current(h, firstOfCall); }
+int enqueue_node(dnl_handle *h, const StepTail &tail) { return launch_node(h, true, tail); }
 int read_time_state(dnl_handle *h, DevTime *t) { return read_time(h, t); }
 
 int launch_gather_raw(int dim, const GatherArgs &g, cudaStream_t s)
@@ -1657,7 +1675,7 @@ int dnl_prologue(dnl_handle *h)
   // computeInternalForces with the initial Current field (:157), then computeTimeStep(True) (:172)
   if ((r = launch_elem(h, h->stream, 1))) return r;
   if ((r = launch_gather(h))) return r;
-  if ((r = launch_time_step_source(h))) return r;
+  if ((r = launch_time_step_source(h, step_tail_args(h, 0)))) return r;
   if ((r = launch_dt(h, DT_FORCE))) return r;
   DevTime t;
   if ((r = read_time(h, &t))) return r;
@@ -1676,7 +1694,7 @@ int dnl_step(dnl_handle *h, int nsteps, int *steps_done)
   const long long inc0 = h->hostIncrement;
   if ((r = launch_dt(h, DT_PRE))) return r;
   for (int s = 0; s < nsteps; s++)
-    if ((r = enqueue_step(h, inc0 + s + 1, s == nsteps - 1))) return r;
+    if ((r = enqueue_step(h, inc0 + s + 1, s == 0, s == nsteps - 1))) return r;
   DevTime t;
   if ((r = read_time(h, &t))) return r;
   if (steps_done) *steps_done = (int)(t.increment - inc0);
@@ -1775,10 +1793,11 @@ static int step_host(dnl_handle *h, const dnl_state_view *in, int nsteps, dnl_st
       CK(cudaEventRecord(h->ioEv[2], io));
       CK(cudaStreamWaitEvent(s, h->ioEv[2], 0));
     } else {
-      if (bc && (r = launch_bc_current(h))) return r;
+      if ((r = launch_bc_current(h, k == 0))) return r;
       if ((r = launch_elem(h, s, 1))) return r;
     }
-    if ((r = launch_node(h, true))) return r;
+    const int mode = last ? DT_POST : (DT_POST | DT_PRE);
+    if ((r = launch_node(h, true, node_tail(h, incAfter, mode)))) return r;
     h->cur = 1 - h->cur;
     if (last && out) {  // the download, beside the time step's computation
       CK(cudaEventRecord(h->ioEv[1], s));
@@ -1792,8 +1811,7 @@ static int step_host(dnl_handle *h, const dnl_state_view *in, int nsteps, dnl_st
       for (int f = 0; f < 5; f++)
         if (dst[f]) CK(cudaMemcpyAsync(dst[f], h->stage + f * n3, sizeof(double) * n3, cudaMemcpyDeviceToHost, io));
     }
-    if (incAfter % h->freq == 0 && (r = launch_time_step_source(h))) return r;
-    if ((r = launch_dt(h, last ? DT_POST : (DT_POST | DT_PRE)))) return r;
+    if ((r = launch_step_end(h, incAfter, mode))) return r;
   }
   // the handle's later work waits for the second stream (its staging slots, the Current fields)
   CK(cudaEventRecord(h->ioEv[2], io));
@@ -1851,7 +1869,7 @@ int dnl_step_graph(dnl_handle *h, int nsteps, int *steps_done)
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rr = launch_dt(h, DT_PRE);
-    for (int s = 0; s < nsteps && !rr; s++) rr = enqueue_step(h, inc0 + s + 1, s == nsteps - 1);
+    for (int s = 0; s < nsteps && !rr; s++) rr = enqueue_step(h, inc0 + s + 1, s == 0, s == nsteps - 1);
     cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
     if (rr) return rr;
     if (ce != cudaSuccess) {

@@ -161,5 +161,49 @@ static __device__ void dt_update(DevTime *tm, int mode, int freq, int method, do
   }
 }
 
+// scheduled steps (dnl_sens_run, dnl_adjoint): phase 0 initStep with the scheduled step, 1
+// updateTime, 2 both (updateTime of one step then initStep of the next)
+static __device__ void sched_update(DevTime *tm, const double *dts, int phase)
+{
+  if (tm->status) return;
+  if (phase != 0) tm->currentTime = __dadd_rn(tm->currentTime, tm->timeStep);
+  if (phase != 1) {
+    const double dt = dts[tm->increment];
+    tm->timeStep = dt;
+    tm->nextTime = __dadd_rn(tm->currentTime, dt);
+    tm->increment++;
+  }
+}
+
+// Called by every thread of every block of a kernel once its work is done: the block that arrives
+// last runs the step's time logic, for which every other block has read the time record and written
+// its part.  Saves a launch and the gap before it (about 3.5 us of a step) against a kernel of one
+// thread.  The arrival counter is back at 0 afterwards.  Warp 0 of each block must not have left.
+static __device__ void step_tail(const StepTail &t, DevTime *tm)
+{
+  if (!t.mode && !t.sched) return;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  unsigned last = 0;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&tm->arrived, 1u) + 1u == gridDim.x * gridDim.y;
+    __threadfence();
+  }
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (!last) return;
+  if (threadIdx.x == 0) tm->arrived = 0u;
+  if (t.count) {
+    for (int i = threadIdx.x; i < t.count; i += 32) {
+      const InstParams &p = t.prm[i];
+      dt_update(t.tms + i, t.mode, p.freq, p.method, p.safetyOmega, p.Cs);
+    }
+  } else if (threadIdx.x == 0) {
+    if (t.sched)
+      sched_update(tm, t.dts, t.sched);
+    else
+      dt_update(tm, t.mode, t.freq, t.method, t.safetyOmega, t.Cs);
+  }
+}
 
 }  // namespace dnl

@@ -327,15 +327,17 @@ int sens_run(dnl_handle *h, int nsteps, const double *dts, const SensBatch *bt)
   na.tms = bt ? bt->tms : nullptr;
   const dim3 ngrid((h->N + 255) / 256, kSensParams);
   const int tgrid = (ninst + 127) / 128;
+  StepTail none;  // the tangents' nodal update still reads the time record
+  memset(&none, 0, sizeof none);
   // one step: the primal launches with the scheduled step size, each followed by its tangent
   auto one_step = [&]() -> int {
     int r;
     k_sens_dt<<<tgrid, 128, 0, s>>>(tms, ninst, S->dts, 0);
     launch_counter()++;
     if (bt)
-      r = launch_bc_batch(h, bt->tms, bt->nodeInst);
+      r = launch_bc_batch(h, bt->tms, bt->nodeInst, true);
     else
-      r = enqueue_bc_current(h);
+      r = enqueue_bc_current(h, true);
     if (r) return r;
     if (h->nbcNodes) {
       double **tc = S->tb[h->cur];
@@ -376,9 +378,9 @@ int sens_run(dnl_handle *h, int nsteps, const double *dts, const SensBatch *bt)
     prof_end(h, DNL_PROF_TANGENT, s);
     if (r) return r;
     if (bt)
-      r = launch_node_batch(h, bt->nodeInst, bt->prm, bt->tms);
+      r = launch_node_batch(h, bt->nodeInst, bt->prm, bt->tms, none);
     else
-      r = enqueue_node(h);
+      r = enqueue_node(h, none);
     if (r) return r;
     for (int f = 0; f < 4; f++) {
       na.cur[f] = S->tb[h->cur][f];
