@@ -346,6 +346,7 @@ int dnl_batch_create(int count, const dnl_mesh_desc *meshes, const dnl_material 
     p.alphaM = (2.0 * rb - 1.0) / (1.0 + rb);
     p.beta = (5.0 - 3.0 * rb) / ((1.0 + rb) * (1.0 + rb) * (2.0 - rb));
     p.gamma = 1.5 - p.alphaM;
+    p.ch = node_const(p.alphaM, p.beta, p.gamma);
     const double omegaS = sqrt((12.0 * pow((1 + rb), 3) * (2.0 - rb)) /
                                (10 + 15 * rb - rb * rb + pow(rb, 3) - pow(rb, 4)));
     p.safetyOmega = sps[i].safety * omegaS;

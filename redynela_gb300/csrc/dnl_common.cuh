@@ -361,11 +361,21 @@ struct StepTail {
   const struct InstParams *prm;
 };
 
+// Constants of the Chung-Hulbert update that no step changes: alphaM, 1 - alphaM and its reciprocal,
+// 1/2 - beta, 1 - gamma, beta, gamma
+struct NodeConst {
+  double alphaM, oma, roma, hb, hg, beta, gamma;
+};
+inline NodeConst node_const(double alphaM, double beta, double gamma)
+{
+  return {alphaM, 1.0 - alphaM, 1.0 / (1.0 - alphaM), 0.5 - beta, 1.0 - gamma, beta, gamma};
+}
+
 struct NodeArgs {
   int N, EN;
   const int *start, *entry;
   const double *fe;
-  const double *mass;
+  const double *mass;     // 2N: masses, reciprocals
   NodeFields cur, nxt;
   double *x[3];
   const int *bcIdx;       // per node: -1 or index into bcCode/bcSpeed
@@ -373,13 +383,14 @@ struct NodeArgs {
   const double *bcSpeed;  // 3 per BC node
   double *fint;           // optional [N*DIM] copy of the assembled forces
   DevTime *tm;
-  double alphaM, beta, gamma;
+  NodeConst ch;
   StepTail tail;
 };
 
 // per-instance constants of a batch
 struct InstParams {
   double alphaM, beta, gamma, safetyOmega, Cs;
+  NodeConst ch;
   int freq, method;
 };
 
@@ -440,7 +451,7 @@ struct dnl_handle {
   int *conn;                  // [NEN][E]
   double *x[3];
   int *n2eStart, *n2e;        // node -> element entries
-  double *mass;               // N
+  double *mass;               // 2N: lumped masses, their reciprocals
   // nodal fields, two banks (Node::Current / Node::New swap by index)
   double *fieldMem;
   dnl::NodeFields bank[2];

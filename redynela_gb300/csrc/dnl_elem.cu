@@ -1498,12 +1498,13 @@ __global__ void __launch_bounds__(BLOCK) k_batch_persistent(const __grid_constan
   }
   if (!grid_barrier(a.bar, a.err)) return;
   // ---- assembly + nodal update (k_node_batch)
-  for (int n = tid; n < a.na.N; n += nthreads) {
-    const int i = a.nodeInst[n];
-    const DevTime *tm = a.tms + i;
-    if (tm->done | tm->status) continue;
-    node_update<DIM>(a.na, n, tm->timeStep, a.prm[i].alphaM, a.prm[i].beta, a.prm[i].gamma);
-  }
+  for (int c = 0; c < DIM; c++)
+    for (int n = tid; n < a.na.N; n += nthreads) {
+      const int i = a.nodeInst[n];
+      const DevTime *tm = a.tms + i;
+      if (tm->done | tm->status) continue;
+      node_update<DIM>(a.na, n, c, a.prm[i].ch, node_dt(tm->timeStep, a.prm[i].ch));
+    }
   if (!grid_barrier(a.bar, a.err)) return;
   // ---- Courant lengths of the updated mesh into each instance's minimum (k_courant_batch)
   if (a.courant) {

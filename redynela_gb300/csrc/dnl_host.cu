@@ -36,24 +36,14 @@ namespace {
 
 // ----------------------------------------------------------------------------- gather
 template <int DIM>
-__global__ void __launch_bounds__(256) k_gather(GatherArgs g)
+__global__ void __launch_bounds__(128) k_gather(GatherArgs g)
 {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (n >= g.N) return;
-  const int b = g.start[n], e = g.start[n + 1];
-  double f[DIM];
-#pragma unroll
-  for (int c = 0; c < DIM; c++) f[c] = 0.0;
-  for (int q = b; q < e; q++) {
-    const int ent = __ldg(g.entry + q);
-#pragma unroll
-    for (int c = 0; c < DIM; c++) f[c] = RADD(f[c], __ldg(g.fe + (long)c * g.EN + ent));
-  }
-#pragma unroll
-  for (int c = 0; c < DIM; c++) g.fint[(long)n * DIM + c] = f[c];
+  g.fint[(long)n * DIM + c] = gather_sum(g.fe + (long)c * g.EN, g.entry, g.start[n], g.start[n + 1]);
 }
 
-// scalar gather (mass): out[n] = sum of me entries in ascending element order
+// scalar gather (mass): out[n] = sum of me entries in ascending element order, out[N + n] its reciprocal
 __global__ void __launch_bounds__(256) k_gather1(int N, const int *start, const int *entry,
                                                  const double *me, double *out)
 {
@@ -62,30 +52,33 @@ __global__ void __launch_bounds__(256) k_gather1(int N, const int *start, const 
   double s = 0.;
   for (int q = start[n]; q < start[n + 1]; q++) s = RADD(s, me[entry[q]]);
   out[n] = s;
+  out[(long)N + n] = nr_rcp(s);
 }
 
 // nodal update (node_update, apply_bc) and time-step logic (dt_update): dnl_node.cuh
 
 template <int DIM>
-__global__ void __launch_bounds__(256) k_node(NodeArgs g)
+__global__ void __launch_bounds__(128) k_node(NodeArgs g)
 {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   DevTime *tm = g.tm;
   if (tm->done | tm->status) return;  // set by earlier kernels or by this one's last block: all blocks alike
-  if (n < g.N) node_update<DIM>(g, n, tm->timeStep, g.alphaM, g.beta, g.gamma);
+  const NodeDt k = node_dt_block(tm->timeStep, g.ch);
+  if (n < g.N) node_update<DIM>(g, n, blockIdx.y, g.ch, k);
   step_tail(g.tail, tm);
 }
 
 // batched: node n belongs to instance nodeInst[n] with its own time record and constants
 template <int DIM>
-__global__ void __launch_bounds__(256) k_node_batch(NodeArgs g, const int *nodeInst,
+__global__ void __launch_bounds__(128) k_node_batch(NodeArgs g, const int *nodeInst,
                                                     const InstParams *prm, DevTime *tms)
 {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n < g.N) {
     const int i = nodeInst[n];
     const DevTime *tm = tms + i;
-    if (!(tm->done | tm->status)) node_update<DIM>(g, n, tm->timeStep, prm[i].alphaM, prm[i].beta, prm[i].gamma);
+    if (!(tm->done | tm->status))
+      node_update<DIM>(g, n, blockIdx.y, prm[i].ch, node_dt(tm->timeStep, prm[i].ch));
   }
   step_tail(g.tail, tms);
 }
@@ -329,12 +322,12 @@ GatherArgs gather_args(dnl_handle *h)
 int launch_gather(dnl_handle *h)
 {
   GatherArgs g = gather_args(h);
-  const int grid = (h->N + 255) / 256;
+  const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_gather<2><<<grid, 256, 0, h->stream>>>(g);
+    k_gather<2><<<grid, 128, 0, h->stream>>>(g);
   else
-    k_gather<3><<<grid, 256, 0, h->stream>>>(g);
+    k_gather<3><<<grid, 128, 0, h->stream>>>(g);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -371,15 +364,13 @@ int launch_node(dnl_handle *h, bool keepFint, const StepTail &tail)
   g.bcSpeed = h->bcSpeed;
   g.fint = keepFint ? h->fint : nullptr;
   g.tm = h->tm;
-  g.alphaM = h->alphaM;
-  g.beta = h->beta;
-  g.gamma = h->gamma;
-  const int grid = (h->N + 255) / 256;
+  g.ch = node_const(h->alphaM, h->beta, h->gamma);
+  const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_node<2><<<grid, 256, 0, h->stream>>>(g);
+    k_node<2><<<grid, 128, 0, h->stream>>>(g);
   else
-    k_node<3><<<grid, 256, 0, h->stream>>>(g);
+    k_node<3><<<grid, 128, 0, h->stream>>>(g);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -473,13 +464,13 @@ int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm,
   g.bcSpeed = h->bcSpeed;
   g.fint = h->fint;
   g.tm = nullptr;
-  g.alphaM = g.beta = g.gamma = 0.;
-  const int grid = (h->N + 255) / 256;
+  g.ch = NodeConst{};
+  const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_node_batch<2><<<grid, 256, 0, h->stream>>>(g, nodeInst, prm, tms);
+    k_node_batch<2><<<grid, 128, 0, h->stream>>>(g, nodeInst, prm, tms);
   else
-    k_node_batch<3><<<grid, 256, 0, h->stream>>>(g, nodeInst, prm, tms);
+    k_node_batch<3><<<grid, 128, 0, h->stream>>>(g, nodeInst, prm, tms);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -539,11 +530,11 @@ int read_time_state(dnl_handle *h, DevTime *t) { return read_time(h, t); }
 
 int launch_gather_raw(int dim, const GatherArgs &g, cudaStream_t s)
 {
-  const int grid = (g.N + 255) / 256;
+  const dim3 grid((g.N + 127) / 128, dim);
   if (dim == 2)
-    k_gather<2><<<grid, 256, 0, s>>>(g);
+    k_gather<2><<<grid, 128, 0, s>>>(g);
   else
-    k_gather<3><<<grid, 256, 0, s>>>(g);
+    k_gather<3><<<grid, 128, 0, s>>>(g);
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
@@ -1211,8 +1202,8 @@ int dnl_create(const dnl_mesh_desc *mesh, const dnl_material *mat, const dnl_sol
       }
   }
   CKF(cudaMalloc(&h->stage, sizeof(double) * 15 * (size_t)N));
-  CKF(cudaMalloc(&h->mass, sizeof(double) * N));
-  CKF(cudaMemset(h->mass, 0, sizeof(double) * N));
+  CKF(cudaMalloc(&h->mass, sizeof(double) * 2 * (size_t)N));
+  CKF(cudaMemset(h->mass, 0, sizeof(double) * 2 * (size_t)N));
   // ---- integration points
   const int ncomp = 3 * etype_ns(h->etype) + 3;  // IpLayout::NCOMP
   const int ns = etype_ns(h->etype);

@@ -2,8 +2,8 @@
 // (dnl_host.cu) and the batch's persistent step kernel (dnl_elem.cu):
 //   node_update  the CSR gather of the element forces + ExplicitSolverCH::computePredictions
 //                (ExplicitSolverCH.C:387-431), explicitSolve (:490-545), updateGrid (:555-567) and
-//                the constant boundary conditions (Boundary.C:478-525, 636-665), with the
-//                reference's rounding (__dmul_rn/__dadd_rn in its operation order);
+//                the constant boundary conditions (Boundary.C:478-525, 636-665), in the
+//                reference's operation order, products added by fma;
 //   dt_update    Solver::computeTimeStep (Solver.C:220-267), ExplicitSolverCH::initStep
 //                (:434-447), updateTime and Solver::betweenTimeBounds.
 // Every product and sum is written with an explicit rounding intrinsic or fma, so the code rounds
@@ -15,94 +15,89 @@
 namespace dnl {
 
 // ----------------------------------------------------------------------------- nodal update
-__device__ __forceinline__ void apply_bc(int code, const double *spd, double dt, double cdu[3],
-                                         double ndu[3], double cv[3], double nv[3], double ca[3],
-                                         double na[3])
+// The step's products of the update: dt (1/2 - beta), dt (1 - gamma), dt gamma, dt^2 beta
+struct NodeDt {
+  double dt, c1, c2, cg, cb;
+};
+__device__ __forceinline__ NodeDt node_dt(double dt, const NodeConst &p)
 {
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const int act = (code >> (2 * i)) & 3;
-    if (act == 1) {
-      cdu[i] = ndu[i] = cv[i] = nv[i] = ca[i] = na[i] = 0.;
-    } else if (act == 2) {
-      ca[i] = na[i] = 0.;
-      cv[i] = nv[i] = spd[i];
-      cdu[i] = __dmul_rn(cv[i], dt);
-      ndu[i] = __dmul_rn(nv[i], dt);
-    }
+  return {dt, __dmul_rn(dt, p.hb), __dmul_rn(dt, p.hg), __dmul_rn(dt, p.gamma), __dmul_rn(__dmul_rn(dt, dt), p.beta)};
+}
+// the same for a block that shares one time step, four lanes of its first warp one product each (two
+// FP64 instructions of the pipe instead of five); contains a barrier
+__device__ __forceinline__ NodeDt node_dt_block(double dt, const NodeConst &p)
+{
+  __shared__ double c[4];
+  if (threadIdx.x < 4) {
+    const int l = threadIdx.x;
+    const double f = l == 0 ? p.hb : l == 1 ? p.hg : l == 2 ? p.gamma : p.beta;
+    const double dt2 = __dmul_rn(dt, dt);
+    c[l] = __dmul_rn(l == 3 ? dt2 : dt, f);
   }
+  __syncthreads();
+  return {dt, c[0], c[1], c[2], c[3]};
 }
 
-// one node of the Chung-Hulbert update; dt and the integration constants of its mesh.  In 2D the
-// third components of the nodal fields stay 0 (nothing writes them), so only DIM are read and
-// written.  The two divisions of the corrector, F/M and (. - alphaM a)/(1 - alphaM), go through
-// a reciprocal and one residual correction (quot): the FP64 pipe bounds this kernel too.
-template <int DIM>
-__device__ __forceinline__ void node_update(const NodeArgs &g, int n, double dt, double alphaM,
-                                            double beta, double gamma)
+// sum of the element forces' component fe over a node's slots, in ascending element order; eight
+// slots' loads are in flight at a time (one by one, each add waited for two dependent loads)
+__device__ __forceinline__ double gather_sum(const double *fe, const int *entry, int b, int e)
 {
-  double cdu[3] = {0., 0., 0.}, cv[3] = {0., 0., 0.}, ca[3] = {0., 0., 0.}, cd[3] = {0., 0., 0.};
-  double ndu[3] = {0., 0., 0.}, nv[3] = {0., 0., 0.}, na[3] = {0., 0., 0.}, nd[3] = {0., 0., 0.};
+  double f = 0.0;
+  for (int q = b; q < e; q += 8) {
+    int ent[8];
+    double v[8];
+    const int n = e - q;
 #pragma unroll
-  for (int i = 0; i < DIM; i++) {
-    cdu[i] = g.cur.du[i][n];
-    cv[i] = g.cur.v[i][n];
-    ca[i] = g.cur.a[i][n];
-    cd[i] = g.cur.disp[i][n];
-  }
-  // computePredictions
-  const double c1 = __dmul_rn(dt, __dsub_rn(0.5, beta)), c2 = __dmul_rn(dt, __dsub_rn(1., gamma));
+    for (int k = 0; k < 8; k++) ent[k] = __ldg(entry + q + (k < n ? k : 0));
 #pragma unroll
-  for (int i = 0; i < DIM; i++) {
-    ndu[i] = __dmul_rn(__dadd_rn(__dmul_rn(ca[i], c1), cv[i]), dt);
-    nd[i] = __dadd_rn(cd[i], ndu[i]);
-    nv[i] = __dadd_rn(__dmul_rn(ca[i], c2), cv[i]);
-    na[i] = 0.0;
+    for (int k = 0; k < 8; k++) v[k] = __ldg(fe + ent[k]);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < n) f = __dadd_rn(f, v[k]);
   }
+  return f;
+}
+
+// Component c of node n of the Chung-Hulbert update.  One thread per component: the FP64 pipe bounds
+// this kernel (22 FP64 instructions per component of a node with eight elements, 64 cycles each), and
+// on small meshes its latency, which is a third or half per thread that way.  In 2D the third
+// components of the nodal fields stay 0 (nothing writes them).  Products are added by fma, with one
+// rounding.  Against one thread per node, loads and adds of the gather alternating, masses inverted
+// here: 674,000 nodes of hexahedra 108 -> 96 us, 306 nodes 8.1 -> 5.8 us (of a tetrahedral bar, 24 elements
+// to a node: a step of 47 -> 37 us).  The two
+// divisions of the corrector, F/M and (. - alphaM a)/(1 - alphaM), go through a
+// reciprocal (the mass's is stored beside it) and one residual correction (quot).
+template <int DIM>
+__device__ __forceinline__ void node_update(const NodeArgs &g, int n, int c, const NodeConst &p, const NodeDt &k)
+{
+  double cv = g.cur.v[c][n], ca = g.cur.a[c][n];
+  const double cd = g.cur.disp[c][n], x = g.x[c][n];
+  const double m = g.mass[n], rm = g.mass[(long)g.N + n];
   const int bc = g.bcIdx[n];
-  int code = 0;
-  const double *spd = nullptr;
-  if (bc >= 0) {
-    code = g.bcCode[bc];
-    spd = g.bcSpeed + 3 * bc;
-    apply_bc(code, spd, dt, cdu, ndu, cv, nv, ca, na);
-  }
-  // assembled internal forces of this node
-  double f[DIM];
-#pragma unroll
-  for (int c = 0; c < DIM; c++) f[c] = 0.0;
-  for (int q = g.start[n]; q < g.start[n + 1]; q++) {
-    const int ent = __ldg(g.entry + q);
-#pragma unroll
-    for (int c = 0; c < DIM; c++) f[c] = __dadd_rn(f[c], __ldg(g.fe + (long)c * g.EN + ent));
-  }
-  if (g.fint) {
-#pragma unroll
-    for (int c = 0; c < DIM; c++) g.fint[(long)n * DIM + c] = f[c];
-  }
+  const int act = bc >= 0 ? (g.bcCode[bc] >> (2 * c)) & 3 : 0;  // 1 restrained, 2 imposed speed
+  // computePredictions
+  double ndu = __dmul_rn(fma(ca, k.c1, cv), k.dt);
+  double nv = fma(ca, k.c2, cv);
+  if (act) ca = 0.;
+  // assembled internal forces
+  const double f = gather_sum(g.fe + (long)c * g.EN, g.entry, g.start[n], g.start[n + 1]);
+  if (g.fint) g.fint[(long)n * DIM + c] = f;
   // explicitSolve
-  const double m = g.mass[n], rm = nr_rcp(m);
-#pragma unroll
-  for (int c = 0; c < DIM; c++) na[c] = quot(f[c], m, rm);
-  const double cg = __dmul_rn(dt, gamma), cb = __dmul_rn(__dmul_rn(dt, dt), beta);
-  const double oma = __dsub_rn(1.0, alphaM), roma = nr_rcp(oma);
-#pragma unroll
-  for (int i = 0; i < DIM; i++) {
-    na[i] = __dsub_rn(na[i], __dmul_rn(alphaM, ca[i]));
-    na[i] = quot(na[i], oma, roma);
-    nv[i] = __dadd_rn(nv[i], __dmul_rn(cg, na[i]));
-    ndu[i] = __dadd_rn(ndu[i], __dmul_rn(cb, na[i]));
+  double na = quot(f, m, rm);
+  na = quot(fma(-p.alphaM, ca, na), p.oma, p.roma);
+  nv = fma(k.cg, na, nv);
+  ndu = fma(k.cb, na, ndu);
+  if (act) {
+    const double s = act == 2 ? g.bcSpeed[3 * bc + c] : 0.;
+    na = 0.;
+    nv = s;
+    ndu = act == 2 ? __dmul_rn(s, k.dt) : 0.;
   }
-  if (bc >= 0) apply_bc(code, spd, dt, cdu, ndu, cv, nv, ca, na);
-#pragma unroll
-  for (int i = 0; i < DIM; i++) {
-    nd[i] = __dadd_rn(cd[i], ndu[i]);
-    g.nxt.du[i][n] = ndu[i];
-    g.nxt.v[i][n] = nv[i];
-    g.nxt.a[i][n] = na[i];
-    g.nxt.disp[i][n] = nd[i];
-    g.x[i][n] = __dadd_rn(g.x[i][n], ndu[i]);
-  }
+  g.nxt.du[c][n] = ndu;
+  g.nxt.v[c][n] = nv;
+  g.nxt.a[c][n] = na;
+  g.nxt.disp[c][n] = __dadd_rn(cd, ndu);
+  g.x[c][n] = __dadd_rn(x, ndu);
 }
 
 enum { DT_FORCE = 1, DT_POST = 2, DT_PRE = 4 };
