@@ -75,7 +75,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   for (int k = 0; k < NEN; k++) {
     double fb[DIM];
 #pragma unroll
-    for (int i = 0; i < DIM; i++) fb[i] = __ldg(a.fbar + (long)i * N + node[k]);
+    for (int i = 0; i < DIM; i++) fb[i] = a.fbar[(long)i * N + node[k]];
 #pragma unroll
     for (int l = 0; l < DIM; l++) {
       const double d = SH::dN(pt, k, l);
@@ -502,6 +502,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
 template <int ET>
 __global__ void __launch_bounds__(128) k_elem_adj(AdjElemArgs a)
 {
+  after_previous();
   constexpr int NIP = Elem<ET>::NIP;
   constexpr int EPW = 32 / NIP;
   __shared__ double red[128 / 32][EPW][AdjSlot<ET>::SIZE];
@@ -520,15 +521,15 @@ int launch_elem_adj(int etype, const AdjElemArgs &a, cudaStream_t s)
   const long threads = (long)a.E * etype_nip(etype);
   const int grid = (int)((threads + 127) / 128);
   if (etype == DNL_ELQUA4NAX)
-    k_elem_adj<DNL_ELQUA4NAX><<<grid, 128, 0, s>>>(a);
+    launch_next(k_elem_adj<DNL_ELQUA4NAX>, grid, 128, s, a);
   else if (etype == DNL_ELQUA4N2D)
-    k_elem_adj<DNL_ELQUA4N2D><<<grid, 128, 0, s>>>(a);
+    launch_next(k_elem_adj<DNL_ELQUA4N2D>, grid, 128, s, a);
   else if (etype == DNL_ELHEX8N3D)
-    k_elem_adj<DNL_ELHEX8N3D><<<grid, 128, 0, s>>>(a);
+    launch_next(k_elem_adj<DNL_ELHEX8N3D>, grid, 128, s, a);
   else if (etype == DNL_ELTET4N3D)
-    k_elem_adj<DNL_ELTET4N3D><<<grid, 128, 0, s>>>(a);
+    launch_next(k_elem_adj<DNL_ELTET4N3D>, grid, 128, s, a);
   else
-    k_elem_adj<DNL_ELTET10N3D><<<grid, 128, 0, s>>>(a);
+    launch_next(k_elem_adj<DNL_ELTET10N3D>, grid, 128, s, a);
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
@@ -540,7 +541,7 @@ int launch_elem_tape_raw(int etype, const ElemArgs &a, cudaStream_t s)
   if (!etype_has_sens(etype)) return DNL_ERR_ARG;
   const long threads = (long)a.E * etype_nip(etype);
   const int grid = (int)((threads + 127) / 128);
-  DNL_BY_ETYPE(etype, (k_elem<ET, true><<<grid, 128, 0, s>>>(a)));
+  DNL_BY_ETYPE(etype, (launch_next(k_elem<ET, true>, grid, 128, s, a)));
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }

@@ -94,13 +94,18 @@ void adj_drop_graphs(AdjState *A)
 }
 
 // opens a sequence of scheduled steps (sched_update); the nodal update's last block runs the others
-__global__ void k_adj_dt(DevTime *tm, const double *dts) { sched_update(tm, dts, 0); }
+__global__ void k_adj_dt(DevTime *tm, const double *dts)
+{
+  after_previous();
+  sched_update(tm, dts, 0);
+}
 
 // a step's record: the coordinates (3N), the Current delta_disp (3N) and the integration-point
 // state (n doubles) copied into rec one after another, in one launch
 __global__ void k_adj_record(long N, long nip, const double *x, const double *du, const double *ip,
                              double *rec)
 {
+  after_previous();
   const long total = 6 * N + nip;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x)
     rec[i] = i < 3 * N ? x[i] : (i < 6 * N ? du[i - 3 * N] : ip[i - 6 * N]);
@@ -130,6 +135,7 @@ struct AdjNodeArgs {
 template <int DIM>
 __global__ void __launch_bounds__(256) k_node_adj(AdjNodeArgs g)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= g.N) return;
   const long N = g.N;
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(256) k_gather_adj(int N, int EN, const int *st
                                                     double *lc, const int *bcIdx, const int *bcCode,
                                                     DevTime *tm)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n == 0) tm->increment--;  // the step undone; nothing else in this kernel reads the record
   if (n >= N) return;
@@ -179,8 +186,8 @@ __global__ void __launch_bounds__(256) k_gather_adj(int N, int EN, const int *st
     const int ent = __ldg(entry + q);
 #pragma unroll
     for (int c = 0; c < DIM; c++) {
-      sx[c] += __ldg(xe + (long)c * EN + ent);
-      su[c] += __ldg(ue + (long)c * EN + ent);
+      sx[c] += xe[(long)c * EN + ent];
+      su[c] += ue[(long)c * EN + ent];
     }
   }
   const int bc = bcIdx[n];
@@ -353,15 +360,14 @@ int adj_primal_step(dnl_handle *h, const double *dtsDev, double *rec, double *ta
   cudaStream_t s = h->stream;
   const size_t N = h->N, nIP = ip_total(h);  // one allocation holds every group's state
   if (first) {
-    k_adj_dt<<<1, 1, 0, s>>>(h->tm, dtsDev);
+    launch_next(k_adj_dt, 1, 1, s, h->tm, dtsDev);
     launch_counter()++;
   }
   int r;
   if ((r = enqueue_bc_current(h, first))) return r;
   if (rec) {
     const long total = 6 * (long)N + (long)ip_ncomp(h->etype) * nIP;
-    k_adj_record<<<(unsigned)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096), 256, 0, s>>>(
-        (long)N, (long)ip_ncomp(h->etype) * nIP, h->x[0], h->bank[h->cur].du[0], h->ip, rec);
+    launch_next(k_adj_record, (unsigned)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096), 256, s, (long)N, (long)ip_ncomp(h->etype) * nIP, h->x[0], h->bank[h->cur].du[0], h->ip, rec);
     launch_counter()++;
   }
   // with tapeOut: the same pass (bit for bit) also writing its per-point record there
@@ -453,9 +459,9 @@ int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double
   const int gridN = (h->N + 255) / 256;
   prof_begin(h, s);
   if (h->dim == 2)
-    k_node_adj<2><<<gridN, 256, 0, s>>>(g);
+    launch_next(k_node_adj<2>, gridN, 256, s, g);
   else
-    k_node_adj<3><<<gridN, 256, 0, s>>>(g);
+    launch_next(k_node_adj<3>, gridN, 256, s, g);
   prof_end(h, DNL_PROF_NODE, s);
   launch_counter()++;
   AdjElemArgs aa;
@@ -483,10 +489,10 @@ int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double
   if (r) return r;
   prof_begin(h, s);
   if (h->dim == 2)
-    k_gather_adj<2><<<gridN, 256, 0, s>>>(h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
+    launch_next(k_gather_adj<2>, gridN, 256, s, h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
                                           A->xbar, lc, h->bcIdx, h->bcCode, h->tm);
   else
-    k_gather_adj<3><<<gridN, 256, 0, s>>>(h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
+    launch_next(k_gather_adj<3>, gridN, 256, s, h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
                                           A->xbar, lc, h->bcIdx, h->bcCode, h->tm);
   prof_end(h, DNL_PROF_NODE, s);
   launch_counter()++;

@@ -564,6 +564,40 @@ __device__ __forceinline__ double quot(double a, double b, double r)
   return fma(fma(-q0, b, a), r, q0);
 }
 
+// ------------------------------------------------------------------ dependent launches
+// The kernels of a step follow one another on one stream, a few microseconds each on small meshes, and
+// the gap between two plain launches is about 1.2 us.  Launched by launch_next, a kernel's blocks may
+// become resident while its predecessor's last blocks still run; after_previous, which every such
+// kernel calls before it reads or writes anything (and before any return), waits until the
+// predecessor has completed and its writes are visible, then lets the successor's launch begin.  A
+// grid starts only once all blocks of the one before it have, so a waiting grid takes no place that
+// the running one needs.  Memory copies and plain launches in between order as always.
+// A call of 200 steps of a 5 x 50 axisymmetric bar: 5.31 -> 4.31 ms, 40 steps of 16,000 elements 1.58 ->
+// 1.47 ms.  Under capture the launches stay plain: the edges of a replayed graph are already short, and
+// with dependent ones 20 steps of a batch of 32 bars took 2.57 ms instead of 2.47, an adjoint of 150
+// steps 14.9 instead of 14.6.
+__device__ __forceinline__ void after_previous()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch_next(void (*kernel)(P...), dim3 grid, int block, cudaStream_t s, const A &...args)
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cap);
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.gridDim = grid;
+  c.blockDim = dim3(block);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // CALL instantiated for the handle's element type, as ET (CALL in parentheses when it has commas)
 #define DNL_ET_CASE(etype, T, CALL) \
   if ((etype) == (T)) {             \

@@ -1157,6 +1157,7 @@ constexpr int elem_min_blocks(int et, bool tape, bool general)
 template <int ET, bool TAPE = false, bool GENERAL = false>
 __global__ void __launch_bounds__(128, elem_min_blocks(ET, TAPE, GENERAL)) k_elem(const __grid_constant__ ElemArgs a)
 {
+  after_previous();
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int EPW = 32 / NIP;  // elements per warp
   __shared__ double red[128 / 32][EPW][etype_slots(ET)];
@@ -1183,6 +1184,7 @@ template <int ET, int BLOCK, bool TAPE = false>
 __global__ void __launch_bounds__(BLOCK) k_elem_batch(const __grid_constant__ ElemArgs a, const int *elemInst,
                                                       const Material *mats, DevTime *tms)
 {
+  after_previous();
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int EPW = 32 / NIP;
   __shared__ double red[BLOCK / 32][EPW][etype_slots(ET)];
@@ -1351,6 +1353,7 @@ __device__ __forceinline__ double elem_length(const ElemArgs &a, int e)
 template <int KIND>
 __global__ void __launch_bounds__(256) k_courant(ElemArgs a, StepTail tail)
 {
+  after_previous();
   if (a.tm->done | a.tm->status) return;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double len = 1e300;
@@ -1381,6 +1384,7 @@ __global__ void __launch_bounds__(256) k_courant(ElemArgs a, StepTail tail)
 template <int KIND>
 __global__ void __launch_bounds__(256) k_courant_batch(ElemArgs a, const int *elemInst, DevTime *tms, StepTail tail)
 {
+  after_previous();
   const int eRaw = blockIdx.x * blockDim.x + threadIdx.x;
   if ((eRaw & ~31) >= a.E) return;
   const int e = eRaw < a.E ? eRaw : a.E - 1;
@@ -1625,9 +1629,9 @@ int launch_elem(dnl_handle *h, cudaStream_t s, int gate)
   prof_begin(h, s);
   const bool general = h->elemMat || h->mat.hard.law != DNL_HARD_POWER;
   if (general)
-    DNL_BY_ETYPE(h->etype, (k_elem<ET, false, true><<<grid, 128, 0, s>>>(a)));
+    DNL_BY_ETYPE(h->etype, (launch_next(k_elem<ET, false, true>, grid, 128, s, a)));
   else
-    DNL_BY_ETYPE(h->etype, (k_elem<ET><<<grid, 128, 0, s>>>(a)));
+    DNL_BY_ETYPE(h->etype, (launch_next(k_elem<ET>, grid, 128, s, a)));
   launch_counter()++;
   // further element groups: same pass, their own element type (one material: the power law or
   // the general instance as above)
@@ -1637,9 +1641,9 @@ int launch_elem(dnl_handle *h, cudaStream_t s, int gate)
     b.gate = gate;
     const int gg = (int)(((long)g.E * g.nip + 127) / 128);
     if (general)
-      DNL_BY_ETYPE(g.etype, (k_elem<ET, false, true><<<gg, 128, 0, s>>>(b)));
+      DNL_BY_ETYPE(g.etype, (launch_next(k_elem<ET, false, true>, gg, 128, s, b)));
     else
-      DNL_BY_ETYPE(g.etype, (k_elem<ET><<<gg, 128, 0, s>>>(b)));
+      DNL_BY_ETYPE(g.etype, (launch_next(k_elem<ET>, gg, 128, s, b)));
     launch_counter()++;
   }
   prof_end(h, DNL_PROF_ELEM, s);
@@ -1660,7 +1664,7 @@ int launch_elem_tape(dnl_handle *h, cudaStream_t s, double *tape)
     a.tape = tape + (gi < 0 ? 0 : (long)TapeLayout<DNL_ELHEX8N3D>::NT * h->extra[gi].ipOff);
     const long threads = (long)a.E * etype_nip(et);
     const int grid = (int)((threads + 127) / 128);
-    DNL_BY_ETYPE(et, (k_elem<ET, true><<<grid, 128, 0, s>>>(a)));
+    DNL_BY_ETYPE(et, (launch_next(k_elem<ET, true>, grid, 128, s, a)));
     launch_counter()++;
   }
   prof_end(h, DNL_PROF_ELEM, s);
@@ -1701,7 +1705,7 @@ int launch_elem_batch(int etype, int block, const ElemArgs &a, const int *elemIn
     block = 128;
   const long threads = (long)a.E * etype_nip(etype);
   const int grid = (int)((threads + block - 1) / block);
-#define DNL_EB(ET, B) k_elem_batch<ET, B><<<grid, B, 0, s>>>(a, elemInst, mats, tms)
+#define DNL_EB(ET, B) launch_next(k_elem_batch<ET, B>, grid, B, s, a, elemInst, mats, tms)
   if (etype == DNL_ELHEX8N3D_1PT) {
     if (block == 64) DNL_EB(DNL_ELHEX8N3D_1PT, 64);
     else DNL_EB(DNL_ELHEX8N3D_1PT, 128);
@@ -1735,7 +1739,7 @@ int launch_elem_batch_tape(int etype, const ElemArgs &a, const int *elemInst, co
   if (!etype_has_sens(etype)) return DNL_ERR_ARG;
   const long threads = (long)a.E * etype_nip(etype);
   const int grid = (int)((threads + 127) / 128);
-  DNL_BY_ETYPE(etype, (k_elem_batch<ET, 128, true><<<grid, 128, 0, s>>>(a, elemInst, mats, tms)));
+  DNL_BY_ETYPE(etype, (launch_next(k_elem_batch<ET, 128, true>, grid, 128, s, a, elemInst, mats, tms)));
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
@@ -1755,11 +1759,11 @@ int launch_courant_batch(int etype, const ElemArgs &a, const int *elemInst, DevT
 {
   const int kind = etype_length_kind(etype), grid = (a.E + 255) / 256;
   if (kind == 0)
-    k_courant_batch<0><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
+    launch_next(k_courant_batch<0>, grid, 256, s, a, elemInst, tms, tail);
   else if (kind == 1)
-    k_courant_batch<1><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
+    launch_next(k_courant_batch<1>, grid, 256, s, a, elemInst, tms, tail);
   else
-    k_courant_batch<2><<<grid, 256, 0, s>>>(a, elemInst, tms, tail);
+    launch_next(k_courant_batch<2>, grid, 256, s, a, elemInst, tms, tail);
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
@@ -1779,11 +1783,11 @@ int launch_courant(dnl_handle *h, cudaStream_t s, const StepTail &tail)
     const int kind = etype_length_kind(et), grid = (a.E + 255) / 256;
     const StepTail &t = gi == h->nextra - 1 ? tail : none;  // the last group's kernel ends the step
     if (kind == 0)
-      k_courant<0><<<grid, 256, 0, s>>>(a, t);
+      launch_next(k_courant<0>, grid, 256, s, a, t);
     else if (kind == 1)
-      k_courant<1><<<grid, 256, 0, s>>>(a, t);
+      launch_next(k_courant<1>, grid, 256, s, a, t);
     else
-      k_courant<2><<<grid, 256, 0, s>>>(a, t);
+      launch_next(k_courant<2>, grid, 256, s, a, t);
     launch_counter()++;
   }
   prof_end(h, DNL_PROF_COURANT, s);

@@ -38,6 +38,7 @@ namespace {
 template <int DIM>
 __global__ void __launch_bounds__(128) k_gather(GatherArgs g)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (n >= g.N) return;
   g.fint[(long)n * DIM + c] = gather_sum(g.fe + (long)c * g.EN, g.entry, g.start[n], g.start[n + 1]);
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(256) k_gather1(int N, const int *start, const 
 template <int DIM>
 __global__ void __launch_bounds__(128) k_node(NodeArgs g)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   DevTime *tm = g.tm;
   if (tm->done | tm->status) return;  // set by earlier kernels or by this one's last block: all blocks alike
@@ -73,6 +75,7 @@ template <int DIM>
 __global__ void __launch_bounds__(128) k_node_batch(NodeArgs g, const int *nodeInst,
                                                     const InstParams *prm, DevTime *tms)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n < g.N) {
     const int i = nodeInst[n];
@@ -88,6 +91,7 @@ __global__ void __launch_bounds__(128) k_node_batch(NodeArgs g, const int *nodeI
 __global__ void k_bc_current(int nb, const int *nodes, const int *code, const double *speed,
                              NodeFields cur, DevTime *tmBase, const int *nodeInst)
 {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nb) return;
   const DevTime *tm = tmBase + (nodeInst ? nodeInst[nodes[i]] : 0);
@@ -158,11 +162,13 @@ __global__ void k_bc_current_va(int nb, const int *nodes, const int *code, const
 // ----------------------------------------------------------------------------- time step
 __global__ void k_dt(DevTime *tm, StepTail a)
 {
+  after_previous();
   dt_update(tm, a.mode, a.freq, a.method, a.safetyOmega, a.Cs);
 }
 
 __global__ void k_dt_batch(DevTime *tms, const InstParams *prm, int count, int mode)
 {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   dt_update(tms + i, mode, prm[i].freq, prm[i].method, prm[i].safetyOmega, prm[i].Cs);
@@ -325,9 +331,9 @@ int launch_gather(dnl_handle *h)
   const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_gather<2><<<grid, 128, 0, h->stream>>>(g);
+    launch_next(k_gather<2>, grid, 128, h->stream, g);
   else
-    k_gather<3><<<grid, 128, 0, h->stream>>>(g);
+    launch_next(k_gather<3>, grid, 128, h->stream, g);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -368,9 +374,9 @@ int launch_node(dnl_handle *h, bool keepFint, const StepTail &tail)
   const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_node<2><<<grid, 128, 0, h->stream>>>(g);
+    launch_next(k_node<2>, grid, 128, h->stream, g);
   else
-    k_node<3><<<grid, 128, 0, h->stream>>>(g);
+    launch_next(k_node<3>, grid, 128, h->stream, g);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -379,7 +385,7 @@ int launch_node(dnl_handle *h, bool keepFint, const StepTail &tail)
 int launch_dt(dnl_handle *h, int mode)
 {
   prof_begin(h, h->stream);
-  k_dt<<<1, 1, 0, h->stream>>>(h->tm, step_tail_args(h, mode));
+  launch_next(k_dt, 1, 1, h->stream, h->tm, step_tail_args(h, mode));
   prof_end(h, DNL_PROF_OTHER, h->stream);
   launch_counter()++;
   return check_launch();
@@ -392,9 +398,8 @@ int launch_bc_current(dnl_handle *h, bool firstOfCall)
 {
   if (!h->nbcNodes || (!firstOfCall && !h->hasSpeedBC)) return 0;
   prof_begin(h, h->stream);
-  k_bc_current<<<(h->nbcNodes + 127) / 128, 128, 0, h->stream>>>(h->nbcNodes, h->bcNodeList, h->bcCode,
-                                                                  h->bcSpeed, h->bank[h->cur], h->tm,
-                                                                  nullptr);
+  launch_next(k_bc_current, (h->nbcNodes + 127) / 128, 128, h->stream, h->nbcNodes, h->bcNodeList, h->bcCode,
+              h->bcSpeed, h->bank[h->cur], h->tm, (const int *)nullptr);
   prof_end(h, DNL_PROF_OTHER, h->stream);
   launch_counter()++;
   return check_launch();
@@ -468,9 +473,9 @@ int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm,
   const dim3 grid((h->N + 127) / 128, h->dim);
   prof_begin(h, h->stream);
   if (h->dim == 2)
-    k_node_batch<2><<<grid, 128, 0, h->stream>>>(g, nodeInst, prm, tms);
+    launch_next(k_node_batch<2>, grid, 128, h->stream, g, nodeInst, prm, tms);
   else
-    k_node_batch<3><<<grid, 128, 0, h->stream>>>(g, nodeInst, prm, tms);
+    launch_next(k_node_batch<3>, grid, 128, h->stream, g, nodeInst, prm, tms);
   prof_end(h, DNL_PROF_NODE, h->stream);
   launch_counter()++;
   return check_launch();
@@ -479,7 +484,7 @@ int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm,
 int launch_dt_batch(dnl_handle *h, DevTime *tms, const InstParams *prm, int count, int mode)
 {
   prof_begin(h, h->stream);
-  k_dt_batch<<<(count + 127) / 128, 128, 0, h->stream>>>(tms, prm, count, mode);
+  launch_next(k_dt_batch, (count + 127) / 128, 128, h->stream, tms, prm, count, mode);
   prof_end(h, DNL_PROF_OTHER, h->stream);
   launch_counter()++;
   return check_launch();
@@ -489,7 +494,7 @@ int launch_bc_batch(dnl_handle *h, DevTime *tms, const int *nodeInst, bool first
 {
   if (!h->nbcNodes || (!firstOfCall && !h->hasSpeedBC)) return 0;
   prof_begin(h, h->stream);
-  k_bc_current<<<(h->nbcNodes + 127) / 128, 128, 0, h->stream>>>(h->nbcNodes, h->bcNodeList, h->bcCode,
+  launch_next(k_bc_current, (h->nbcNodes + 127) / 128, 128, h->stream, h->nbcNodes, h->bcNodeList, h->bcCode,
                                                                   h->bcSpeed, h->bank[h->cur], tms,
                                                                   nodeInst);
   prof_end(h, DNL_PROF_OTHER, h->stream);

@@ -50,7 +50,7 @@ __device__ __forceinline__ double gather_sum(const double *fe, const int *entry,
 #pragma unroll
     for (int k = 0; k < 8; k++) ent[k] = __ldg(entry + q + (k < n ? k : 0));
 #pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = __ldg(fe + ent[k]);
+    for (int k = 0; k < 8; k++) v[k] = fe[ent[k]];
 #pragma unroll
     for (int k = 0; k < 8; k++)
       if (k < n) f = __dadd_rn(f, v[k]);

@@ -133,6 +133,7 @@ struct PulseArgs {
 template <int ET>
 __global__ void __launch_bounds__(128) k_pulse_setup(PulseArgs a)
 {
+  after_previous();
   using T = Elem<ET>;
   constexpr int NIP = T::NIP, NEN = T::NEN, DIM = T::DIM;
   constexpr bool AXI = ET == DNL_ELQUA4NAX, TWO_D = DIM == 2;
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(128) k_pulse_setup(PulseArgs a)
 template <int ET>
 __global__ void __launch_bounds__(128) k_pulse_kx(PulseArgs a)
 {
+  after_previous();
   using T = Elem<ET>;
   constexpr int NIP = T::NIP, NEN = T::NEN, DIM = T::DIM;
   constexpr bool AXI = ET == DNL_ELQUA4NAX;
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(128) k_pulse_kx(PulseArgs a)
 template <int DIM>
 __global__ void __launch_bounds__(256) k_pulse_gather(PulseArgs a, int EN)
 {
+  after_previous();
   DevTime *tm = a.tm;
   if (tm->done | tm->status | tm->pulseDone) return;
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -449,6 +452,7 @@ __global__ void __launch_bounds__(256) k_pulse_gather(PulseArgs a, int EN)
 
 __global__ void k_pulse_check(DevTime *tm, int maxIt)
 {
+  after_previous();
   if (tm->done | tm->status | tm->pulseDone) return;
   const double fmax = __longlong_as_double((long long)tm->pulseMaxBits);
   tm->pulseMaxBits = 0ull;
@@ -481,6 +485,7 @@ int &pulse_cap()
 
 __global__ void k_pulse_begin(DevTime *tm)
 {
+  after_previous();
   if (tm->done | tm->status) return;
   tm->pulseDone = 0;
   tm->pulseIter = 0;
@@ -547,25 +552,25 @@ int launch_pulse(dnl_handle *h, cudaStream_t s)
   }
   auto gridOf = [](const ElemGroup &g) { return (int)(((long)g.E * g.nip + 127) / 128); };
   prof_begin(h, s);
-  k_pulse_begin<<<1, 1, 0, s>>>(h->tm);
-  DNL_BY_ETYPE(h->etype, (k_pulse_setup<ET><<<gridIP, 128, 0, s>>>(a)));
+  launch_next(k_pulse_begin, 1, 1, s, h->tm);
+  DNL_BY_ETYPE(h->etype, (launch_next(k_pulse_setup<ET>, gridIP, 128, s, a)));
   for (int gi = 0; gi < h->nextra; gi++)
-    DNL_BY_ETYPE(h->extra[gi].etype, (k_pulse_setup<ET><<<gridOf(h->extra[gi]), 128, 0, s>>>(ga[gi])));
+    DNL_BY_ETYPE(h->extra[gi].etype, (launch_next(k_pulse_setup<ET>, gridOf(h->extra[gi]), 128, s, ga[gi])));
   prof_end(h, DNL_PROF_PULSE, s);
   launch_counter() += 2 + h->nextra;
   const int batch = 4;
   for (int round = 0; round < (pulse_cap() + batch) / batch + 1; round++) {
     for (int b = 0; b < batch; b++) {
       prof_begin(h, s);
-      DNL_BY_ETYPE(h->etype, (k_pulse_kx<ET><<<gridIP, 128, 0, s>>>(a)));
+      DNL_BY_ETYPE(h->etype, (launch_next(k_pulse_kx<ET>, gridIP, 128, s, a)));
       for (int gi = 0; gi < h->nextra; gi++)
-        DNL_BY_ETYPE(h->extra[gi].etype, (k_pulse_kx<ET><<<gridOf(h->extra[gi]), 128, 0, s>>>(ga[gi])));
+        DNL_BY_ETYPE(h->extra[gi].etype, (launch_next(k_pulse_kx<ET>, gridOf(h->extra[gi]), 128, s, ga[gi])));
       if (h->dim == 2) {
-        k_pulse_gather<2><<<gridN, 256, 0, s>>>(a, (int)h->EN);
+        launch_next(k_pulse_gather<2>, gridN, 256, s, a, (int)h->EN);
       } else {
-        k_pulse_gather<3><<<gridN, 256, 0, s>>>(a, (int)h->EN);
+        launch_next(k_pulse_gather<3>, gridN, 256, s, a, (int)h->EN);
       }
-      k_pulse_check<<<1, 1, 0, s>>>(h->tm, pulse_cap());
+      launch_next(k_pulse_check, 1, 1, s, h->tm, pulse_cap());
       prof_end(h, DNL_PROF_PULSE, s);
       launch_counter() += 3 + h->nextra;
     }

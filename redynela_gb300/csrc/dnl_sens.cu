@@ -54,6 +54,7 @@ namespace {
 
 __global__ void k_sens_dt(DevTime *tms, int count, const double *dts, int phase)
 {
+  after_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   DevTime *tm = tms + i;
@@ -106,6 +107,7 @@ struct SensNodeArgs {
 template <int DIM>
 __global__ void __launch_bounds__(256) k_node_tan(SensNodeArgs g)
 {
+  after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   const int dir = blockIdx.y;
   if (n >= g.N) return;
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(256) k_node_tan(SensNodeArgs g)
   for (int q = g.start[n]; q < g.start[n + 1]; q++) {
     const int ent = __ldg(g.entry + q);
 #pragma unroll
-    for (int c = 0; c < DIM; c++) f[c] += __ldg(fe + (long)c * g.EN + ent);
+    for (int c = 0; c < DIM; c++) f[c] += fe[(long)c * g.EN + ent];
   }
   // the tangents need no correctly rounded quotients: reciprocals (nr_rcp) times the numerators
   const double rm = nr_rcp(g.mass[n]);
@@ -332,7 +334,7 @@ int sens_run(dnl_handle *h, int nsteps, const double *dts, const SensBatch *bt)
   // one step: the primal launches with the scheduled step size, each followed by its tangent
   auto one_step = [&]() -> int {
     int r;
-    k_sens_dt<<<tgrid, 128, 0, s>>>(tms, ninst, S->dts, 0);
+    launch_next(k_sens_dt, tgrid, 128, s, tms, ninst, S->dts, 0);
     launch_counter()++;
     if (bt)
       r = launch_bc_batch(h, bt->tms, bt->nodeInst, true);
@@ -388,13 +390,13 @@ int sens_run(dnl_handle *h, int nsteps, const double *dts, const SensBatch *bt)
     }
     prof_begin(h, s);
     if (h->dim == 2)
-      k_node_tan<2><<<ngrid, 256, 0, s>>>(na);
+      launch_next(k_node_tan<2>, ngrid, 256, s, na);
     else
-      k_node_tan<3><<<ngrid, 256, 0, s>>>(na);
+      launch_next(k_node_tan<3>, ngrid, 256, s, na);
     prof_end(h, DNL_PROF_NODE, s);
     launch_counter()++;
     h->cur = 1 - h->cur;
-    k_sens_dt<<<tgrid, 128, 0, s>>>(tms, ninst, S->dts, 1);
+    launch_next(k_sens_dt, tgrid, 128, s, tms, ninst, S->dts, 1);
     launch_counter()++;
     return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
   };

@@ -585,6 +585,7 @@ __device__ __forceinline__ void elem_tan(const SensElemArgs &a, int e, int dir, 
 template <int ET>
 __global__ void __launch_bounds__(128) k_elem_tan(SensElemArgs a)
 {
+  after_previous();
   constexpr int NIP = Elem<ET>::NIP, NEN = Elem<ET>::NEN, DIM = Elem<ET>::DIM;
   constexpr int GPW = 32 / NIP;  // (element, direction) groups per warp
   __shared__ double red[128 / 32][GPW][NIP * NEN * DIM];
@@ -605,7 +606,7 @@ int launch_elem_tan(int etype, const SensElemArgs &a, cudaStream_t s)
   if (!etype_has_sens(etype)) return DNL_ERR_ARG;
   const long threads = (long)a.E * kSensParams * etype_nip(etype);
   const int grid = (int)((threads + 127) / 128);
-  DNL_BY_ETYPE(etype, (k_elem_tan<ET><<<grid, 128, 0, s>>>(a)));
+  DNL_BY_ETYPE(etype, (launch_next(k_elem_tan<ET>, grid, 128, s, a)));
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
 }
