@@ -687,7 +687,7 @@ int dnl_adjoint_forward(dnl_handle *h, int ckpt_stride, double *coords)
     cudaStream_t s = h->stream;
     k_aos3<<<(unsigned)((h->N + 255) / 256), 256, 0, s>>>(h->N, h->x[0], A->fbar);
     launch_counter()++;
-    CKA(cudaMemcpyAsync(coords, A->fbar, sizeof(double) * 3 * (size_t)h->N, cudaMemcpyDeviceToHost, s));
+    CKA(copy_out(coords, A->fbar, sizeof(double) * 3 * (size_t)h->N, s));
     CKA(cudaStreamSynchronize(s));
   }
   return 0;
@@ -757,7 +757,7 @@ int dnl_run_schedule(dnl_handle *h, int nsteps, const double *dts, double *coord
   if (coords) {
     k_aos3<<<(unsigned)((h->N + 255) / 256), 256, 0, s>>>(h->N, h->x[0], A->runOut);
     launch_counter()++;
-    CKA(cudaMemcpyAsync(coords, A->runOut, sizeof(double) * 3 * (size_t)h->N, cudaMemcpyDeviceToHost, s));
+    CKA(copy_out(coords, A->runOut, sizeof(double) * 3 * (size_t)h->N, s));
   }
   CKA(cudaStreamSynchronize(s));
   h->hostIncrement = t.increment;

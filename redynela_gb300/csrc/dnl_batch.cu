@@ -190,6 +190,16 @@ __global__ void k_batch_evpn(long nIP, int nip, const int *elemInst, const Mater
   evpn[i] = pow(evp[i], mats[elemInst[i / nip]].n);
 }
 
+// coordinates of one instance's nodes, node-major
+__global__ void k_batch_coords(int n, const double *x, const double *y, const double *z, double *out)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  out[3L * i] = x[i];
+  out[3L * i + 1] = y[i];
+  out[3L * i + 2] = z[i];
+}
+
 // the launches of nsteps steps from increment inc0 in the batch's mode
 int enqueue_steps(dnl_batch *b, long long inc0, int nsteps)
 {
@@ -740,12 +750,12 @@ int dnl_batch_get_coords(dnl_batch *b, int inst, double *coords)
   if (!b || !coords || inst < 0 || inst >= b->count) return DNL_ERR_ARG;
   dnl_handle *h = b->h;
   const int n0 = b->nodeOff[inst], n1 = b->nodeOff[inst + 1];
-  std::vector<double> c(n1 - n0);
+  double *out = h->stage + 3 * (size_t)n0;
+  k_batch_coords<<<(n1 - n0 + 255) / 256, 256, 0, h->stream>>>(n1 - n0, h->x[0] + n0, h->x[1] + n0, h->x[2] + n0, out);
+  launch_counter()++;
+  BK(cudaGetLastError());
+  BK(copy_out(coords, out, sizeof(double) * 3 * (size_t)(n1 - n0), h->stream));
   BK(cudaStreamSynchronize(h->stream));
-  for (int r = 0; r < 3; r++) {
-    BK(cudaMemcpy(c.data(), h->x[r] + n0, sizeof(double) * (n1 - n0), cudaMemcpyDeviceToHost));
-    for (int n = 0; n < n1 - n0; n++) coords[3 * (size_t)n + r] = c[n];
-  }
   return 0;
 }
 
@@ -753,10 +763,9 @@ int dnl_batch_get_fint(dnl_batch *b, int inst, double *fint)
 {
   if (!b || !fint || inst < 0 || inst >= b->count) return DNL_ERR_ARG;
   dnl_handle *h = b->h;
+  BK(copy_out(fint, h->fint + (size_t)h->dim * b->nodeOff[inst],
+              sizeof(double) * h->dim * (b->nodeOff[inst + 1] - b->nodeOff[inst]), h->stream));
   BK(cudaStreamSynchronize(h->stream));
-  BK(cudaMemcpy(fint, h->fint + (size_t)h->dim * b->nodeOff[inst],
-                sizeof(double) * h->dim * (b->nodeOff[inst + 1] - b->nodeOff[inst]),
-                cudaMemcpyDeviceToHost));
   return 0;
 }
 

@@ -564,6 +564,17 @@ __device__ __forceinline__ double quot(double a, double b, double r)
   return fma(fma(-q0, b, a), r, q0);
 }
 
+// ------------------------------------------------------------------ copies to the caller's arrays
+// make_present has the kernel map an array's missing pages at once, contents unchanged; copy_out is
+// cudaMemcpyAsync from the device after that.  The pages of a fresh array do not exist yet, and a copy
+// from the device that meets them faults once a page: reading back the nodal fields of 225,000 nodes
+// (16 MB) into fresh arrays took 13.2 ms, 6.0 with the pages touched one by one, 0.85-1.0 mapped by
+// one call, 0.4 into pages that exist.  Page-locked memory needs nothing.
+namespace dnl {
+void make_present(void *dst, size_t bytes);
+cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s);
+}
+
 // ------------------------------------------------------------------ dependent launches
 // The kernels of a step follow one another on one stream, a few microseconds each on small meshes, and
 // the gap between two plain launches is about 1.2 us.  Launched by launch_next, a kernel's blocks may

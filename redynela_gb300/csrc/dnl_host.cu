@@ -21,6 +21,9 @@
 #include <cstring>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <nvtx3/nvToolsExt.h>
 
 #include "dnl_common.cuh"
@@ -450,6 +453,26 @@ int enqueue_step(dnl_handle *h, long long incAfter, bool first, bool last)
 }  // namespace
 
 namespace dnl {
+void make_present(void *dst, size_t bytes)
+{
+#ifdef MADV_POPULATE_WRITE
+  cudaPointerAttributes at;
+  if (bytes < 4096 || cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) return;
+  static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t first = (uintptr_t)dst / page * page;
+  // no effect on pages that are there; where it is refused the copy meets the pages as it finds them
+  (void)madvise((void *)first, (uintptr_t)dst + bytes - first, MADV_POPULATE_WRITE);
+#else
+  (void)dst, (void)bytes;
+#endif
+}
+
+cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s)
+{
+  make_present(dst, bytes);
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+}
+
 int launch_node_batch(dnl_handle *h, const int *nodeInst, const InstParams *prm, DevTime *tms,
                       const StepTail &tail)
 {
@@ -1560,10 +1583,9 @@ int dnl_get_state(dnl_handle *h, dnl_state_view *s)
   if ((r = transpose_set(h, fs, false, h->stream))) return r;
   for (int f = 0; f < 5; f++)
     if (out[f])
-      CK(cudaMemcpyAsync(out[f], h->stage + (size_t)f * 3 * N, sizeof(double) * 3 * (size_t)N,
-                         cudaMemcpyDeviceToHost, h->stream));
+      CK(copy_out(out[f], h->stage + (size_t)f * 3 * N, sizeof(double) * 3 * (size_t)N, h->stream));
+  if (s->mass) CK(copy_out(s->mass, h->mass, sizeof(double) * N, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (s->mass) CK(cudaMemcpy(s->mass, h->mass, sizeof(double) * N, cudaMemcpyDeviceToHost));
   if (!(s->S || s->Eps || s->EpsPlas || s->p || s->evp || s->Sig)) return 0;
   const int ns = etype_ns(h->etype);  // the same for every group of a domain (one family)
   const int I0[6] = {0, 1, 2, 0, 0, 1}, I1[6] = {0, 1, 2, 1, 2, 2};
@@ -1572,6 +1594,7 @@ int dnl_get_state(dnl_handle *h, dnl_state_view *s)
     std::vector<double> ib(nIP), pb(nIP);
     auto getT = [&](double *dst, int base, const double *addP) -> int {
       dst += 9 * o;
+      make_present(dst, sizeof(double) * 9 * nIP);
       for (size_t i = 0; i < 9 * nIP; i++) dst[i] = 0.;
       for (int k = 0; k < ns; k++) {
         CK(cudaMemcpy(ib.data(), g.ip + (size_t)(base + k) * nIP, sizeof(double) * nIP, cudaMemcpyDeviceToHost));
@@ -1591,7 +1614,10 @@ int dnl_get_state(dnl_handle *h, dnl_state_view *s)
     if (s->p || s->Sig) CK(cudaMemcpy(pb.data(), g.ip + (size_t)(3 * ns) * nIP, sizeof(double) * nIP, cudaMemcpyDeviceToHost));
     if (s->p) memcpy(s->p + o, pb.data(), sizeof(double) * nIP);
     if (s->Sig && (r = getT(s->Sig, 0, pb.data()))) return r;
-    if (s->evp) CK(cudaMemcpy(s->evp + o, g.ip + (size_t)(3 * ns + 1) * nIP, sizeof(double) * nIP, cudaMemcpyDeviceToHost));
+    if (s->evp) {
+      CK(copy_out(s->evp + o, g.ip + (size_t)(3 * ns + 1) * nIP, sizeof(double) * nIP, h->stream));
+      CK(cudaStreamSynchronize(h->stream));
+    }
   }
   return 0;
 }
@@ -1616,8 +1642,8 @@ int dnl_get_step_tensors(dnl_handle *h, double *dEps, double *R)
 int dnl_get_fint(dnl_handle *h, double *fint)
 {
   if (!h || !fint) return DNL_ERR_ARG;
+  CK(copy_out(fint, h->fint, sizeof(double) * (size_t)h->dim * h->N, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  CK(cudaMemcpy(fint, h->fint, sizeof(double) * (size_t)h->dim * h->N, cudaMemcpyDeviceToHost));
   return 0;
 }
 
@@ -1643,7 +1669,10 @@ int dnl_internal_forces(dnl_handle *h, const double *coords, const double *du, d
   DevTime t;
   if ((r = read_time(h, &t))) return r;
   if (t.status) return t.status;
-  if (fint) CK(cudaMemcpy(fint, h->fint, sizeof(double) * (size_t)h->dim * h->N, cudaMemcpyDeviceToHost));
+  if (fint) {
+    CK(copy_out(fint, h->fint, sizeof(double) * (size_t)h->dim * h->N, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+  }
   return 0;
 }
 
@@ -1805,7 +1834,7 @@ static int step_host(dnl_handle *h, const dnl_state_view *in, int nsteps, dnl_st
         if (dst[f]) add_field(h, fs, f);
       if ((r = transpose_set(h, fs, false, io))) return r;
       for (int f = 0; f < 5; f++)
-        if (dst[f]) CK(cudaMemcpyAsync(dst[f], h->stage + f * n3, sizeof(double) * n3, cudaMemcpyDeviceToHost, io));
+        if (dst[f]) CK(copy_out(dst[f], h->stage + f * n3, sizeof(double) * n3, io));
     }
     if ((r = launch_step_end(h, incAfter, mode))) return r;
   }

@@ -461,15 +461,14 @@ int sens_outputs(dnl_handle *h, double *coords, double *dcoords)
   const int grid = (h->N + 255) / 256;
   if (coords) {
     k_to_nodes<<<grid, 256, 0, s>>>(h->N, S->out, h->x[0], h->x[1], h->x[2]);
-    CKS(cudaMemcpyAsync(coords, S->out, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
+    CKS(copy_out(coords, S->out, sizeof(double) * 3 * N, s));
     CKS(cudaStreamSynchronize(s));
   }
   if (dcoords)
     for (int dir = 0; dir < kSensParams; dir++) {
       const double *b = S->tx + (long)dir * 3 * N;
       k_to_nodes<<<grid, 256, 0, s>>>(h->N, S->out, b, b + N, b + 2 * N);
-      CKS(cudaMemcpyAsync(dcoords + (long)dir * 3 * N, S->out, sizeof(double) * 3 * N,
-                          cudaMemcpyDeviceToHost, s));
+      CKS(copy_out(dcoords + (long)dir * 3 * N, S->out, sizeof(double) * 3 * N, s));
       CKS(cudaStreamSynchronize(s));
     }
   return 0;
