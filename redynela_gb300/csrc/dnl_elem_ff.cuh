@@ -394,37 +394,42 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     tape(TL::DETJ, f64_of(det, DIM * j20));
     tape(TL::RAD, AXI ? f64_of(Rad) : 0.);
     tape(TL::VRR, AXI ? f64_of(G[2][2]) : 0.);
-    double lv[3], lg[3], il[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      lv[k] = f64_add(1., lam[k]);
-      lg[k] = scale2<-1>(ln_eig(lv[k]));
-      il[k] = rsqrt(lv[k]);
-    }
 #pragma unroll
     for (int k = 0; k < 9; k++) {
       const int i = k / 3, j = k % 3;
-      tape(TL::F + k, f64_add(i == j ? 1. : 0., G[i][j]));
-      tape(TL::R + k, f64_add(i == j ? 1. : 0., Q[i][j]));
+      const double d = i == j ? 1. : 0.;
+      const bool out = TWO_D && (i == 2) != (j == 2);  // outside the plane case's blocks: 0
+      tape(TL::F + k, out ? 0. : f64_add(d, G[i][j]));
+      tape(TL::R + k, out ? 0. : f64_add(d, Q[i][j]));
       tape(TL::V + k, f64_of(V[i][j]));
+    }
+    // divided differences of ln(l)/2 and l^-1/2 (Daleckii-Krein factors), l = 1 + lam; the second is
+    // -1 / (sqrt(li lj) (sqrt(li) + sqrt(lj))).  Between the plane case's blocks they multiply zeros.  In FP64,
+    // with divisions and logarithms, they and the sums that are 0 took a quarter of this pass on 4,000
+    // axisymmetric elements (its adjoint of 150 steps: 13.3 -> 12.5 ms).
+    ff il[3], sq[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const ff y = ff_add(ff{1.f, 0.f}, lam[k]);
+      il[k] = ff_add(ff{1.f, 0.f}, rsqrt1p_ff(lam[k]));
+      sq[k] = ff_mul(y, il[k]);
     }
 #pragma unroll
     for (int k = 0; k < 6; k++) {
       const int i = sym_i(k), j = sym_j(k);
-      // divided differences of ln(l)/2 and l^-1/2 (Daleckii-Krein factors)
-      double g, hh;
+      const bool out = TWO_D && k > 3;
+      ff g = zero, hh = zero;
       if (i == j) {
-        g = 0.5 * il[i] * il[i];
-        hh = -0.5 * il[i] * il[i] * il[i];
-      } else {
-        const double li = lv[i], lj = lv[j];
-        const double mean = 0.5 * (li + lj), q = (li - lj) / mean;
-        g = fabs(q) < 1e-3 ? 0.5 * fma(q * q, fma(q * q, 1. / 80., 1. / 12.), 1.) / mean : (lg[i] - lg[j]) / (li - lj);
-        hh = -il[i] * il[j] / fma(li, il[i], lj * il[j]);
+        const ff h = ff_scale(ff_mul(il[i], il[i]), 0.5f);
+        g = h;
+        hh = ff_neg(ff_mul(h, il[i]));
+      } else if (!out) {
+        g = half_log_slope_ff(lam[i], lam[j]);
+        hh = ff_neg(ff_mul(ff_mul(il[i], il[j]), ff_rcp(ff_add(sq[i], sq[j]))));
       }
-      tape(TL::GD + k, g);
-      tape(TL::HD + k, hh);
-      tape(TL::UI + k, f64_add(i == j ? 1. : 0., H[k]));
+      tape(TL::GD + k, f64_of(g));
+      tape(TL::HD + k, f64_of(hh));
+      tape(TL::UI + k, out ? 0. : f64_add(i == j ? 1. : 0., H[k]));
     }
   } else {
     conv = strain_ff<TWO_D, false>(G, E, mge, c_tolFF.polar, c_caps[0], first, Ln, Q);

@@ -330,6 +330,16 @@ FFD ff half_log1p_ff(ff x)
   const ff s = ff_mul(x, ff_rcp(ff_add(ff{2.f, 0.f}, x)));
   return ff_mul(s, atanh_series_ff(s));
 }
+// (ln(1 + a) - ln(1 + b)) / (2 (a - b)), 1 / (2 (1 + a)) in the limit, |a|, |b| <= 0.4: with w = 2 + a + b and
+// u = (a - b) / w it is atanh(u) / (u w), no difference of logarithms; where u is beyond the series the
+// logarithms are apart enough to be subtracted
+FFD ff half_log_slope_ff(ff a, ff b)
+{
+  const ff d = ff_sub(a, b), rw = ff_rcp(ff_add(ff{2.f, 0.f}, ff_add(a, b)));
+  const ff u = ff_mul(d, rw);
+  if (f_abs(u.h) <= 0.17f) return ff_mul(atanh_series_ff(u), rw);
+  return ff_mul(ff_sub(half_log1p_ff(a), half_log1p_ff(b)), ff_rcp(d));
+}
 FFD ff rsqrt1p_ff(ff x)
 {
   const ff y = ff_add(ff{1.f, 0.f}, x);
