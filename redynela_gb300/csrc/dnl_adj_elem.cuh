@@ -500,13 +500,14 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
 }
 
 template <int ET>
-__global__ void __launch_bounds__(128) k_elem_adj(AdjElemArgs a)
+__global__ void __launch_bounds__(128) k_elem_adj(const __grid_constant__ AdjElemArgs a)
 {
   after_previous();
   constexpr int NIP = Elem<ET>::NIP;
   constexpr int EPW = 32 / NIP;
   __shared__ double red[128 / 32][EPW][AdjSlot<ET>::SIZE];
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a.tm && gtid == 0) a.tm->increment--;  // nothing in this kernel reads the record
   if ((gtid & ~31) / NIP >= a.E) return;
   const int eRaw = gtid / NIP;
   const bool valid = eRaw < a.E;

@@ -16,8 +16,9 @@
 //      - the adjoint of the nodal update (k_node_adj): Chung-Hulbert corrector and predictor and
 //        the constant boundary conditions, whose formulas are linear in the state,
 //      - the adjoint of the element pass (k_elem_adj), and
-//      - the reverse gather (k_gather_adj): each node sums its element nodes' coordinate and
-//        delta_disp adjoints in ascending element order, no atomics.
+//      - the reverse gather (k_node_adj too, in one launch with the nodal update's adjoint of the step
+//        undone next): each node sums its element nodes' coordinate and delta_disp adjoints in
+//        ascending element order, no atomics.
 //    The hardening parameters' derivatives accumulate per integration point over the steps; the
 //    initial velocity's is the adjoint of the first step's Current velocity along v0's direction.
 //
@@ -112,96 +113,81 @@ __global__ void k_adj_record(long N, long nip, const double *x, const double *du
 }
 
 struct AdjNodeArgs {
-  int N;
-  const double *mass;
+  int N, EN;
+  const int *start, *entry;
+  const double *xe, *ue;  // element nodes' adjoints of the coordinates and of delta_disp
+  const double *mass;     // 2N: masses, reciprocals
   const int *bcIdx, *bcCode;
-  const double *ln;  // adjoints of the New field after the step, [du, v, a, disp][3][N]
-  double *lc;        // adjoints of the Current field before it (v, a, disp written here)
-  const double *xbar;
+  double *ln;        // adjoints of the New field after the step whose node update is undone, [du, v, a, disp][3][N]:
+                     // of the Current field before the step whose gather is reversed
+  double *lc;        // adjoints of the Current field before the former step (v, a, disp written here)
+  double *xbar;
   double *fbar;
   const double *dts; // the schedule; the step undone is the time record's increment - 1
   const DevTime *tm;
-  double alphaM, beta, gamma;
+  NodeConst ch;
 };
 
-// Adjoint of node_update (dnl_host.cu) for one node.  Per free component, with
-// u = adj(New du) + adj(New disp) + adj(x') (delta_disp feeds the New field, the displacement and
-// the coordinates) and a' = adj(New a) + dt gamma adj(New v) + dt^2 beta u:
+// Reverse gather of one step (GATHER) and the adjoint of the nodal update of the step before it (NODE),
+// component c = blockIdx.y of one node a thread: between two reverse steps both are one launch, as
+// nothing but the node's own component passes from one to the other (a launch and a gap of some 2.5 us
+// less per step, and the adjoints of the fields between them stay in registers).
+//
+// GATHER: adj(x) += sum of the element nodes' coordinate adjoints, adj(Current du) = sum of their
+// delta_disp adjoints (ascending element order, as k_gather); then the constant boundary conditions,
+// which overwrite the Current du, v, a of their components before the element pass reads them
+// (k_bc_current), zero those components' adjoints.
+//
+// NODE: adjoint of node_update.  Per free component, with u = adj(New du) + adj(New disp) + adj(x')
+// (delta_disp feeds the New field, the displacement and the coordinates) and a' = adj(New a) +
+// dt gamma adj(New v) + dt^2 beta u:
 //   adj(F) = a' / (m (1 - alphaM)),
 //   adj(Current a) = -alphaM / (1 - alphaM) a' + dt (1 - gamma) adj(New v) + dt^2 (1/2 - beta) u,
 //   adj(Current v) = adj(New v) + dt u,  adj(Current disp) = adj(New disp).
 // A restrained or imposed-speed component's New du, v, a are constants: no force or Current
 // velocity / acceleration adjoint from it.
-template <int DIM>
-__global__ void __launch_bounds__(256) k_node_adj(AdjNodeArgs g)
+template <bool GATHER, bool NODE>
+__global__ void __launch_bounds__(128) k_node_adj(const __grid_constant__ AdjNodeArgs g)
 {
   after_previous();
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (n >= g.N) return;
-  const long N = g.N;
+  const long N = g.N, o = c * N + n;
   const int bc = g.bcIdx[n];
-  const int code = bc >= 0 ? g.bcCode[bc] : 0;
-  const double dt = g.dts[g.tm->increment - 1];
-  const double rm = 1.0 / g.mass[n], roma = 1.0 / (1.0 - g.alphaM);
-  const double c1 = dt * (0.5 - g.beta), c2 = dt * (1.0 - g.gamma);
-  const double cg = dt * g.gamma, cb = dt * dt * g.beta;
-#pragma unroll
-  for (int i = 0; i < DIM; i++) {
-    const long o = (long)i * N + n;
-    const double nu = g.ln[o], nv = g.ln[3 * N + o], na = g.ln[6 * N + o], nd = g.ln[9 * N + o];
-    const double u = nu + nd + g.xbar[o];
+  const bool fixed = bc >= 0 && ((g.bcCode[bc] >> (2 * c)) & 3);
+  double xb = g.xbar[o], nu = 0., nv = 0., na = 0.;
+  if (GATHER) {
+    const int b = g.start[n], e = g.start[n + 1];
+    xb += gather_sum(g.xe + (long)c * g.EN, g.entry, b, e);
+    nu = gather_sum(g.ue + (long)c * g.EN, g.entry, b, e);
+    if (fixed) nu = 0.;
+    g.xbar[o] = xb;
+    if (!NODE) {
+      g.ln[o] = nu;
+      if (fixed) g.ln[3 * N + o] = g.ln[6 * N + o] = 0.;
+    }
+  } else {
+    nu = g.ln[o];
+  }
+  if (NODE) {
+    if (!(GATHER && fixed)) {
+      nv = g.ln[3 * N + o];
+      na = g.ln[6 * N + o];
+    }
+    const double nd = g.ln[9 * N + o];
+    const double dt = g.dts[g.tm->increment - 1], rm = g.mass[N + n];
+    const double u = nu + nd + xb;
     double fb = 0., cv = 0., ca = 0.;
-    if (!((code >> (2 * i)) & 3)) {
-      const double ab = fma(cb, u, fma(cg, nv, na));
-      fb = ab * rm * roma;
-      ca = fma(-g.alphaM * roma, ab, fma(c2, nv, dt * c1 * u));
+    if (!fixed) {
+      const double ab = fma(dt * dt * g.ch.beta, u, fma(dt * g.ch.gamma, nv, na));
+      fb = ab * rm * g.ch.roma;
+      ca = fma(-g.ch.alphaM * g.ch.roma, ab, fma(dt * g.ch.hg, nv, dt * (dt * g.ch.hb) * u));
       cv = fma(dt, u, nv);
     }
     g.fbar[o] = fb;
     g.lc[3 * N + o] = cv;
     g.lc[6 * N + o] = ca;
     g.lc[9 * N + o] = nd;
-  }
-}
-
-// Reverse gather: adj(x) += sum of the element nodes' coordinate adjoints, adj(Current du) = sum of
-// their delta_disp adjoints (ascending element order, as k_gather); then the constant boundary
-// conditions, which overwrite the Current du, v, a of their components before the element pass
-// reads them (k_bc_current), zero those components' adjoints.  The time record's increment steps
-// back to the step undone next, whose size the next k_node_adj reads from the schedule.
-template <int DIM>
-__global__ void __launch_bounds__(256) k_gather_adj(int N, int EN, const int *start, const int *entry,
-                                                    const double *xe, const double *ue, double *xbar,
-                                                    double *lc, const int *bcIdx, const int *bcCode,
-                                                    DevTime *tm)
-{
-  after_previous();
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n == 0) tm->increment--;  // the step undone; nothing else in this kernel reads the record
-  if (n >= N) return;
-  double sx[DIM], su[DIM];
-#pragma unroll
-  for (int c = 0; c < DIM; c++) sx[c] = su[c] = 0.;
-  for (int q = start[n]; q < start[n + 1]; q++) {
-    const int ent = __ldg(entry + q);
-#pragma unroll
-    for (int c = 0; c < DIM; c++) {
-      sx[c] += xe[(long)c * EN + ent];
-      su[c] += ue[(long)c * EN + ent];
-    }
-  }
-  const int bc = bcIdx[n];
-  const int code = bc >= 0 ? bcCode[bc] : 0;
-#pragma unroll
-  for (int c = 0; c < DIM; c++) {
-    const long o = (long)c * N + n;
-    xbar[o] += sx[c];
-    const bool fixed = (code >> (2 * c)) & 3;
-    lc[o] = fixed ? 0. : su[c];
-    if (fixed) {
-      lc[3L * N + o] = 0.;
-      lc[6L * N + o] = 0.;
-    }
   }
 }
 
@@ -409,10 +395,11 @@ int adj_restore(dnl_handle *h, AdjState *A, int seg)
 
 // undo one step from its record: its per-point record (kept from the recomputation in `tape`, or
 // regenerated by running the pass again on the step's stored state), then the adjoints of the
-// nodal update, the element pass and the gather; ln / lc: the New / Current nodal adjoints; ipOut:
-// the integration-point state after the step (with a kept record)
-int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double *ln, double *lc,
-                     const double *tape = nullptr, const double *ipOut = nullptr)
+// nodal update (the first step's here, the others' with the gather of the step undone before), the
+// element pass and the gather; ln / lc: the New / Current nodal adjoints; ipOut: the
+// integration-point state after the step (with a kept record); first, last: of a sequence
+int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, double *ln, double *lc, const double *tape,
+                     const double *ipOut, bool first, bool last)
 {
   cudaStream_t s = h->stream;
   const size_t N = h->N, nIP = A->nIP;
@@ -444,6 +431,11 @@ int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double
   }
   AdjNodeArgs g;
   g.N = h->N;
+  g.EN = (int)h->EN;
+  g.start = h->n2eStart;
+  g.entry = h->n2e;
+  g.xe = A->xe;
+  g.ue = A->ue;
   g.mass = h->mass;
   g.bcIdx = h->bcIdx;
   g.bcCode = h->bcCode;
@@ -453,17 +445,14 @@ int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double
   g.fbar = A->fbar;
   g.dts = A->dts;
   g.tm = h->tm;
-  g.alphaM = h->alphaM;
-  g.beta = h->beta;
-  g.gamma = h->gamma;
-  const int gridN = (h->N + 255) / 256;
-  prof_begin(h, s);
-  if (h->dim == 2)
-    launch_next(k_node_adj<2>, gridN, 256, s, g);
-  else
-    launch_next(k_node_adj<3>, gridN, 256, s, g);
-  prof_end(h, DNL_PROF_NODE, s);
-  launch_counter()++;
+  g.ch = node_const(h->alphaM, h->beta, h->gamma);
+  const dim3 gridN((h->N + 127) / 128, h->dim);
+  if (first) {
+    prof_begin(h, s);
+    launch_next(k_node_adj<false, true>, gridN, 128, s, g);
+    prof_end(h, DNL_PROF_NODE, s);
+    launch_counter()++;
+  }
   AdjElemArgs aa;
   aa.N = h->N;
   for (int c = 0; c < 3; c++) aa.x[c] = rec + c * N;
@@ -483,17 +472,18 @@ int adj_reverse_step(dnl_handle *h, AdjState *A, const double *rec, const double
     aa.xe = A->xe + feOff;
     aa.ue = A->ue + feOff;
     aa.gpar = A->gpar + ipOff;
+    aa.tm = gi < 0 ? h->tm : nullptr;
     r = launch_elem_adj(gi < 0 ? h->etype : h->extra[gi].etype, aa, s);
   }
   prof_end(h, DNL_PROF_TANGENT, s);
   if (r) return r;
   prof_begin(h, s);
-  if (h->dim == 2)
-    launch_next(k_gather_adj<2>, gridN, 256, s, h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
-                                          A->xbar, lc, h->bcIdx, h->bcCode, h->tm);
+  g.ln = lc;
+  g.lc = ln;
+  if (last)
+    launch_next(k_node_adj<true, false>, gridN, 128, s, g);
   else
-    launch_next(k_gather_adj<3>, gridN, 256, s, h->N, (int)h->EN, h->n2eStart, h->n2e, A->xe, A->ue,
-                                          A->xbar, lc, h->bcIdx, h->bcCode, h->tm);
+    launch_next(k_node_adj<true, true>, gridN, 128, s, g);
   prof_end(h, DNL_PROF_NODE, s);
   launch_counter()++;
   return cudaPeekAtLastError() == cudaSuccess ? 0 : DNL_ERR_CUDA;
@@ -514,7 +504,7 @@ int adj_segment(dnl_handle *h, AdjState *A, int kind, int len, int &nw)
         const double *tape = A->tapes ? A->tapes + j * A->tapeDoubles : nullptr;
         const double *ipOut = j < len - 1 ? A->slot + (j + 1) * A->slotDoubles + 6 * (size_t)h->N : h->ip;
         if ((r = adj_reverse_step(h, A, A->slot + j * A->slotDoubles, A->lam[nw], A->lam[1 - nw], tape,
-                                  tape ? ipOut : nullptr)))
+                                  tape ? ipOut : nullptr, j == len - 1, j == 0)))
           return r;
         nw = 1 - nw;
       }

@@ -337,6 +337,8 @@ struct AdjElemArgs {
   long feStride;          // element-node slots of the handle's element groups (E*NEN with one type)
   double *gpar;           // [3][gStride]: d L / d(A, B, n) accumulated per integration point
   long gStride;           // integration points of the handle's element groups (E*NIP with one type)
+  DevTime *tm;            // its increment steps back to the step undone next, whose size the next nodal
+                          // adjoint reads from the schedule (nullptr: another element group's launch does it)
   Material mat;
 };
 

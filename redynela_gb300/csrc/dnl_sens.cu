@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) k_node_tan(SensNodeArgs g)
     for (int c = 0; c < DIM; c++) f[c] += fe[(long)c * g.EN + ent];
   }
   // the tangents need no correctly rounded quotients: reciprocals (nr_rcp) times the numerators
-  const double rm = nr_rcp(g.mass[n]);
+  const double rm = g.mass[N + n];
 #pragma unroll
   for (int c = 0; c < DIM; c++) na[c] = f[c] * rm;
   const double cg = dt * gamma, cb = dt * dt * beta, roma = nr_rcp(1. - alphaM);
