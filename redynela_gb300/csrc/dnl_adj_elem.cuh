@@ -131,7 +131,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   for (int i = 0; i < DIM; i++) {
     pb += Sigb[i][i];
 #pragma unroll
-    for (int j = 0; j < DIM; j++) GS[i][j] = fma(0.5, Sigb[i][j] + Sigb[j][i], GS[i][j]);
+    for (int j = i; j < DIM; j++) GS[i][j] = GS[j][i] = i == j ? GS[i][i] + Sigb[i][i] : fma(0.5, Sigb[i][j] + Sigb[j][i], GS[i][j]);
   }
   double detJb = 0., Radb = 0.;
   if (AXI) {
@@ -146,38 +146,23 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   }
 
   // ---- RFI: adj(X) = R^T adj(X') R, adj(R) += 2 adj(X') X' R for S, Eps, EpsPlas
-  double R[3][3], Rb[3][3];
+  double R[3][3], Rb[3][3], GX[3][3];  // GX: the three tensors' sum of adj(X') X'
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       R[i][j] = tp(TL::R + i * 3 + j);
-      Rb[i][j] = 0.;
+      GX[i][j] = 0.;
     }
   auto rfi_adj = [&](double G[3][3], const double X2[3][3]) {
-    double GX[3][3];  // adj(X') X'
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        double s = 0.;
-        if (!zero(i, j)) {
-#pragma unroll
-          for (int k = 0; k < 3; k++)
-            if (!zero(i, k) && !zero(k, j)) s = fma(G[i][k], X2[k][j], s);
-        }
-        GX[i][j] = s;
-      }
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
       for (int j = 0; j < 3; j++) {
         if (zero(i, j)) continue;
-        double s = 0.;
 #pragma unroll
         for (int k = 0; k < 3; k++)
-          if (!zero(i, k) && !zero(k, j)) s = fma(GX[i][k], R[k][j], s);
-        Rb[i][j] = fma(2.0, s, Rb[i][j]);
+          if (!zero(i, k) && !zero(k, j)) GX[i][j] = fma(G[i][k], X2[k][j], GX[i][j]);
       }
     double T1[3][3];  // adj(X') R
 #pragma unroll
@@ -207,6 +192,19 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   rfi_adj(GS, S2);
   rfi_adj(GE, E2);
   rfi_adj(GP, P2);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      double s = 0.;
+      if (!zero(i, j)) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (!zero(i, k) && !zero(k, j)) s = fma(GX[i][k], R[k][j], s);
+        s = 2.0 * s;
+      }
+      Rb[i][j] = s;
+    }
 
   // ---- element-mean pressure: adj(tr dEps) of this point = K / NIP sum over the element's adj(p')
   double trb = 0.;
@@ -227,35 +225,37 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   double gA = 0., gB = 0., gN = 0.;
   if (gam > 0.) {
     const double normS = tp(TL::NORMS), xv = tp(TL::XV), xn = tp(TL::XN), rnorm = nr_rcp(normS);
-    double nh[3][3];
-    symload(nh, [&](int k) { return tp(TL::STR + k) * rnorm; });
-    double gsn = 0., gpn = 0.;
+    // symmetric tensors by their NS components (in the plane case the others are 0): the inner product is
+    // that of the diagonals plus twice that of the rest
+    double nh[NS], nb[NS];
 #pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int k = 0; k < NS; k++) nh[k] = tp(TL::STR + k) * rnorm;
+    auto inner = [&](auto get) {
+      double d = 0., o = 0.;
 #pragma unroll
-      for (int j = 0; j < 3; j++) {
-        gsn = fma(GS[i][j], nh[i][j], gsn);
-        gpn = fma(GP[i][j], nh[i][j], gpn);
+      for (int k = 0; k < NS; k++) {
+        if (k < 3)
+          d = fma(get(k), nh[k], d);
+        else
+          o = fma(get(k), nh[k], o);
       }
+      return fma(2., o, d);
+    };
+    const double gsn = inner([&](int k) { return GS[I0[k]][I1[k]]; });
+    const double gpn = inner([&](int k) { return GP[I0[k]][I1[k]]; });
     // S = Str - 2 G gamma n, EpsPlas += gamma n, evp += sqrt(2/3) gamma, n = Str / |Str|
     const double gamb = fma(-m.G2, gsn, fma(kSqrt23, evpb, gpn));
-    double nb[3][3], nbn = 0.;
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        nb[i][j] = gam * fma(-m.G2, GS[i][j], GP[i][j]);
-        nbn = fma(nb[i][j], nh[i][j], nbn);
-      }
+    for (int k = 0; k < NS; k++) nb[k] = gam * fma(-m.G2, GS[I0[k]][I1[k]], GP[I0[k]][I1[k]]);
+    const double nbn = inner([&](int k) { return nb[k]; });
     const double h = m.nB * xn * nr_rcp(xv);  // n B xv^(n-1)
     const double D = fma(kSqrt23, h, m.dfun0);
     const double lam = gamb * nr_rcp(D);
     // d gamma = (sqrt(3/2) d|Str| - h d evp - d sigma_y / d p) / D
-    const double cn = kSqrt32 * lam;
+    const double cn = fma(-rnorm, nbn, kSqrt32 * lam);
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) GStr[i][j] = fma(cn, nh[i][j], fma(rnorm, fma(-nbn, nh[i][j], nb[i][j]), GS[i][j]));
+    for (int k = 0; k < NS; k++)
+      GStr[I0[k]][I1[k]] = GStr[I1[k]][I0[k]] = fma(cn, nh[k], fma(rnorm, nb[k], GS[I0[k]][I1[k]]));
     evp0b = fma(-h, lam, evpb);
     gA = -lam;
     gB = -lam * xn;
@@ -266,11 +266,11 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
   double GL[3][3];
   {
     const double tg = (GStr[0][0] + GStr[1][1] + GStr[2][2]) * (1.0 / 3.0);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++)
-        GL[i][j] = fma(m.G2, i == j ? GStr[i][j] - tg : GStr[i][j], GE[i][j]) + (i == j ? trb : 0.);
+    const double off = fma(-m.G2, tg, trb);
+    symload(GL, [&](int k) {
+      const double v = fma(m.G2, GStr[I0[k]][I1[k]], GE[I0[k]][I1[k]]);
+      return k < 3 ? v + off : v;
+    });
   }
 
   // ---- the state before the pass: adj(S) = adj(Str), adj(Eps) = adj(Eps'), adj(EpsPlas), p, evp
@@ -309,15 +309,12 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
         }
         T1[i][j] = s;
       }
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) GU_[i][j] = 0.5 * (T1[i][j] + T1[j][i]);
+    symload(GU_, [&](int k) { return k < 3 ? T1[k][k] : 0.5 * (T1[I0[k]][I1[k]] + T1[I1[k]][I0[k]]); });
   }
   double V[3][3];
 #pragma unroll
   for (int k = 0; k < 9; k++) V[k / 3][k % 3] = tp(TL::V + k);
-  double Cb[3][3];
+  double Cb[3][3];  // twice adj(C)
   {
     // A = V^T G V for both adjoints, B = GD o A1 + HD o A2, adj(C) = V B V^T
     double T1[3][3], T2[3][3];  // G V
@@ -348,7 +345,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
             s2 = fma(V[k][i], T2[k][j], s2);
           }
       }
-      Bm[i][j] = Bm[j][i] = fma(tp(TL::GD + q), s1, tp(TL::HD + q) * s2);
+      Bm[i][j] = Bm[j][i] = zero(i, j) ? 0. : fma(tp(TL::GD + q), s1, tp(TL::HD + q) * s2);
     }
     double T3[3][3];  // V B
 #pragma unroll
@@ -370,7 +367,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
         for (int l = 0; l < 3; l++)
           if (!zero(i, l) && !zero(j, l)) s = fma(T3[i][l], V[j][l], s);
       }
-      Cb[i][j] = Cb[j][i] = s;
+      Cb[i][j] = Cb[j][i] = zero(i, j) ? 0. : s + s;
     }
   }
   // adj(F) = 2 F adj(C) + adj(R) U^-1
@@ -387,7 +384,7 @@ __device__ __forceinline__ void elem_adj(const AdjElemArgs &a, int e, int pt, bo
         if (!zero(i, j)) {
 #pragma unroll
           for (int k = 0; k < 3; k++)
-            if (!zero(i, k) && !zero(k, j)) s = fma(2.0 * F[i][k], Cb[k][j], fma(Rb[i][k], Ui[k][j], s));
+            if (!zero(i, k) && !zero(k, j)) s = fma(F[i][k], Cb[k][j], fma(Rb[i][k], Ui[k][j], s));
         }
         Fb[i][j] = s;
       }
