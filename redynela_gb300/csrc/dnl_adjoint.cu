@@ -337,7 +337,7 @@ int adj_alloc(dnl_handle *h, AdjState *A, int nsteps, int stride)
 
 // one scheduled explicit step of the handle (the launches of dnl_sens_run's primal); with `rec`,
 // the coordinates, the Current delta_disp and the integration-point state the element pass reads
-// are copied there first
+// are copied there first (with tapeOut by that pass itself)
 // `first`: the step opens with initStep; `last`: it ends with updateTime; between two steps of a
 // sequence the nodal update's last block does both (the same operations in the same order)
 int adj_primal_step(dnl_handle *h, const double *dtsDev, double *rec, double *tapeOut = nullptr,
@@ -351,13 +351,14 @@ int adj_primal_step(dnl_handle *h, const double *dtsDev, double *rec, double *ta
   }
   int r;
   if ((r = enqueue_bc_current(h, first))) return r;
-  if (rec) {
+  if (rec && !tapeOut) {
     const long total = 6 * (long)N + (long)ip_ncomp(h->etype) * nIP;
-    launch_next(k_adj_record, (unsigned)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096), 256, s, (long)N, (long)ip_ncomp(h->etype) * nIP, h->x[0], h->bank[h->cur].du[0], h->ip, rec);
+    launch_next(k_adj_record, (unsigned)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096), 256, s, (long)N,
+                (long)ip_ncomp(h->etype) * nIP, h->x[0], h->bank[h->cur].du[0], h->ip, rec);
     launch_counter()++;
   }
   // with tapeOut: the same pass (bit for bit) also writing its per-point record there
-  if ((r = tapeOut ? launch_elem_tape(h, s, tapeOut) : launch_elem(h, s, 1))) return r;
+  if ((r = tapeOut ? launch_elem_tape(h, s, tapeOut, rec) : launch_elem(h, s, 1))) return r;
   StepTail tail;
   memset(&tail, 0, sizeof tail);
   tail.sched = last ? 1 : 2;

@@ -291,6 +291,9 @@ struct ElemArgs {
   double *detJ;        // [E*NIP] (written)
   double *stepT;       // optional dEps|R per IP, [18][E*NIP] or nullptr
   double *tape;        // [TapeLayout::NT][E*NIP], written by the tape instance of k_elem
+  // optional, the tape instance: what the pass reads is stored there first, the coordinates and
+  // delta_disp ([6][N], x[0] and du[0] being the first of three arrays of N) and the points' state
+  double *recNodes, *recIp;
   DevTime *tm;
   Material mat;
   const int *elemMat;       // several materials: material of each element (mats), or nullptr
@@ -633,7 +636,7 @@ inline void launch_next(void (*kernel)(P...), dim3 grid, int block, cudaStream_t
 namespace dnl {
 // launchers implemented in dnl_elem.cu
 int launch_elem(dnl_handle *h, cudaStream_t s, int gate);
-int launch_elem_tape(dnl_handle *h, cudaStream_t s, double *tape);
+int launch_elem_tape(dnl_handle *h, cudaStream_t s, double *tape, double *rec = nullptr);
 int launch_elem_tan(int etype, const SensElemArgs &a, cudaStream_t s);
 int launch_elem_batch_tape(int etype, const ElemArgs &a, const int *elemInst, const Material *mats,
                            DevTime *tms, cudaStream_t s);
