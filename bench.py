@@ -43,25 +43,12 @@ from redynela_gb300 import meshes  # noqa: E402
 # of the workload
 ELEM_TRAFFIC_BYTES_PER_ELEMENT = 308.85e6 / 126400
 
-# FP64 thread-instructions of one k_elem<ElHex8n3D> launch per Gauss point in the timed window of
-# the 505,600-element bar (t = 10 us, increment 1,553), from ncu's
-# sm__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum counters of that launch
-# (2,145,155,470 / 573,527,287 / 914,639,971 over the launch's 4,044,800 points, one counter per
-# capture, each a one-pass capture)
-HEX_FP64_INSTR_PER_POINT = {"dfma": 2145155470 / 4044800, "dadd": 573527287 / 4044800,
-                            "dmul": 914639971 / 4044800}
-HEX_FP64_SOURCE = "the 505,600-element bar's timed window (t = 10 us, increment 1,553)"
-
-
-def hex_fp64_flops_per_point() -> float:
-    """FP64 flops per Gauss point (a DFMA counted as two)."""
-    c = HEX_FP64_INSTR_PER_POINT
-    return 2 * c["dfma"] + c["dadd"] + c["dmul"]
-
-
-def hex_fp64_instr_per_point() -> float:
-    c = HEX_FP64_INSTR_PER_POINT
-    return c["dfma"] + c["dadd"] + c["dmul"]
+# Instructions of one k_elem<ElHex8n3D> launch (the pass in pairs of FP32 numbers), from ncu's
+# smsp__inst_executed.sum on the bar cut to 60 layers of elements (606,720 points, early in the impact):
+# warp instructions per warp of 32 points; and the FP64 pipe's share of its peak there
+HEX_WARP_INSTR_PER_WARP = 177184265 / 18960
+HEX_FP64_PIPE_FRAC = 0.108
+HEX_INSTR_SOURCE = "75,840 hexahedra (40 x 40 x 60 layers) after 26 steps of the impact, ncu"
 
 
 def workload(name: str, layers: int = 400):
@@ -209,16 +196,12 @@ def sm_count(device: int = 0) -> int:
     return int(torch.cuda.get_device_properties(device).multi_processor_count)
 
 
-def fp64_roofline(model, launch_s, clocks, device: int = 0):
+def issue_roofline(model, launch_s, clocks, device: int = 0):
     """Roofline of one k_elem launch of `model` taking `launch_s` seconds (CUDA events).
 
-    Bound: the FP64 pipe.  achieved = FP64 flops per launch (the counted mix per Gauss point, a
-    DFMA as two) / launch time, against the DFMA peak measured at the start of this run on this
-    GPU (`dnl_measure_fp64_peak`: independent DFMA chains on every SM); the same launch as FP64
-    instructions issued per second against the pipe's issue ceiling (2 FP64 thread-instructions per
-    SM per cycle at the sampled SM clock).  HBM: the algorithmic bytes per launch over the launch
-    time against the measured copy bandwidth, and the DRAM traffic ncu counted."""
-    from redynela_gb300 import dynela
+    Bound: instruction issue.  achieved = warp instructions per launch (the counted number per warp of
+    Gauss points) / launch time, against four per SM and cycle at the sampled SM clock.  HBM: the
+    algorithmic bytes per launch over the launch time against the measured copy bandwidth."""
     hbm_peak, peak_src = peak_hbm()
     bytes_per_launch = elem_bytes(model)
     traffic = (ELEM_TRAFFIC_BYTES_PER_ELEMENT * model.E) if model.etype == meshes.ELHEX8N3D else None
@@ -231,24 +214,16 @@ def fp64_roofline(model, launch_s, clocks, device: int = 0):
     if model.etype != meshes.ELHEX8N3D or not launch_s:
         return dict(hbm, bound="hbm", kernel=kernel, avg_launch_ms=launch_s * 1e3 if launch_s else None)
     points = model.E * model.nip
-    dfma_peak = dynela.fp64_peak_tflops()
-    achieved = hex_fp64_flops_per_point() * points / launch_s / 1e12
+    achieved = HEX_WARP_INSTR_PER_WARP * points / 32 / launch_s / 1e9
     sms = sm_count(device)
     mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 0.0
-    ceiling = sms * 2.0 * mhz * 1e6  # FP64 thread-instructions per second
-    issued = hex_fp64_instr_per_point() * points / launch_s
-    return {"bound": "fp64", "achieved": achieved, "peak": dfma_peak, "unit": "TFLOP/s",
-            "frac": achieved / dfma_peak if dfma_peak else None, "traffic": traffic,
+    peak = sms * 4.0 * mhz * 1e-3  # 10^9 warp instructions per second
+    return {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "G warp instructions/s",
+            "frac": achieved / peak if peak else None, "traffic": traffic,
             "kernel": kernel, "avg_launch_ms": launch_s * 1e3,
-            "peak_source": "measured on this GPU at the start of the run (DFMA loop); "
-                           "MEASURED_PEAKS.json has no FP64 figure",
-            "flops_per_gauss_point": hex_fp64_flops_per_point(),
-            "fp64_instructions_per_gauss_point": dict(HEX_FP64_INSTR_PER_POINT),
-            "counted_on": HEX_FP64_SOURCE,
-            "issue": {"achieved_instr_per_s": issued, "ceiling_instr_per_s": ceiling,
-                      "frac": issued / ceiling if ceiling else None, "sms": sms,
-                      "sm_mhz": mhz, "per_sm_per_cycle": 2},
-            "hbm": hbm}
+            "peak_source": "4 per SM and cycle at the sampled SM clock",
+            "warp_instructions_per_warp": HEX_WARP_INSTR_PER_WARP, "fp64_pipe_frac_counted": HEX_FP64_PIPE_FRAC,
+            "counted_on": HEX_INSTR_SOURCE, "sms": sms, "sm_mhz": mhz, "hbm": hbm}
 
 
 def run_cpu_baseline(model, sample_desc, min_seconds=10.0, max_steps=400, threads=None,
@@ -375,7 +350,7 @@ def main_ours(args):
     # ---- roofline of the dominant kernel (k_elem): the FP64 pipe binds it, HBM is reported beside
     elem_ms, elem_n = prof["elem"]
     launch_s = elem_ms / elem_n * 1e-3 if elem_n else None
-    roofline = fp64_roofline(model, launch_s, clocks, local)
+    roofline = issue_roofline(model, launch_s, clocks, local)
     kernel_share = {k: round(v[0] / ms, 4) for k, v in prof.items() if v[1]}
 
     # ---- end to end through the C ABI with page-locked host buffers, over the same increments as
