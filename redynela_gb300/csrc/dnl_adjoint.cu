@@ -130,8 +130,8 @@ struct AdjNodeArgs {
 
 // Reverse gather of one step (GATHER) and the adjoint of the nodal update of the step before it (NODE),
 // component c = blockIdx.y of one node a thread: between two reverse steps both are one launch, as
-// nothing but the node's own component passes from one to the other (a launch and a gap of some 2.5 us
-// less per step, and the adjoints of the fields between them stay in registers).
+// nothing but the node's own component passes from one to the other (a launch and a gap, 2 us, less
+// per step, and the adjoints of the fields between them stay in registers).
 //
 // GATHER: adj(x) += sum of the element nodes' coordinate adjoints, adj(Current du) = sum of their
 // delta_disp adjoints (ascending element order, as k_gather); then the constant boundary conditions,
