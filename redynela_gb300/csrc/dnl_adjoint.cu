@@ -118,8 +118,8 @@ struct AdjNodeArgs {
   const double *xe, *ue;  // element nodes' adjoints of the coordinates and of delta_disp
   const double *mass;     // 2N: masses, reciprocals
   const int *bcIdx, *bcCode;
-  double *ln;        // adjoints of the New field after the step whose node update is undone, [du, v, a, disp][3][N]:
-                     // of the Current field before the step whose gather is reversed
+  double *ln;        // adjoints of the New field after the step whose nodal update is undone,
+                     // [du, v, a, disp][3][N]: of the Current field before the step whose gather is reversed
   double *lc;        // adjoints of the Current field before the former step (v, a, disp written here)
   double *xbar;
   double *fbar;

@@ -63,10 +63,10 @@ __device__ __forceinline__ double gather_sum(const double *fe, const int *entry,
 // on small meshes its latency, which is a third or half per thread that way.  In 2D the third
 // components of the nodal fields stay 0 (nothing writes them).  Products are added by fma, with one
 // rounding.  Against one thread per node, loads and adds of the gather alternating, masses inverted
-// here: 539,000 nodes of hexahedra 108 -> 96 us, a step of 306 nodes and 250 quads 30.5 -> 26.4 us (of a tetrahedral bar, 24 elements
-// to a node: a step of 47 -> 37 us).  The two
-// divisions of the corrector, F/M and (. - alphaM a)/(1 - alphaM), go through a
-// reciprocal (the mass's is stored beside it) and one residual correction (quot).
+// here: 539,000 nodes of hexahedra 108 -> 96 us, a step of 306 nodes and 250 quads 30.5 -> 26.4 us,
+// a step of a tetrahedral bar, 24 elements to a node, 47 -> 37 us.  The two divisions of the
+// corrector, F/M and (. - alphaM a)/(1 - alphaM), go through a reciprocal (the mass's is stored
+// beside it) and one residual correction (quot).
 template <int DIM>
 __device__ __forceinline__ void node_update(const NodeArgs &g, int n, int c, const NodeConst &p, const NodeDt &k)
 {
