@@ -824,8 +824,10 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         q[k][r] = ff_sub(q[k][r], t);
       }
     }
-    // a_h = coefficient rho c V^(2/3) / 4 over 2^k, V = 8 detJ
-    const ff ah = ff_mul(ff_mul(mf.rhoCs4, ff_of(a.hourglass)), pow23_ff(ff_scale(det, 8.f)));
+    // a_h = coefficient rho c V^(2/3) / 4 over 2^k, V = 8 detJ; the volume's sign does not matter
+    // (an element that is turned inside out or numbered the other way round is no error in 3D)
+    const ff vol = ff_scale(det.h < 0.f ? ff_neg(det) : det, 8.f);
+    const ff ah = ff_mul(ff_mul(mf.rhoCs4, ff_of(a.hourglass)), pow23_ff(vol));
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       ff P[3], F[8];
