@@ -76,18 +76,29 @@ __device__ __forceinline__ void walsh8(ff (&v)[8])
 }
 // node k's place: bit 0, 1, 2 set where xi, eta, zeta = +1
 __device__ __forceinline__ constexpr int sign_place(int k) { return ((k ^ (k >> 1)) & 1) | (k & 2) | (k & 4); }
-// The transform of a nodal field relative to its value at the element's first node.  The sign
-// product of the directions in m at node b is (-1)^|m| (-1)^popcount(m & b).
-__device__ __forceinline__ void walsh_rel(const double *f, const int (&nd)[8], uint32_t &top, ff (&w)[8])
+// A nodal field relative to its value at the element's first node (d[0] = 0); the high word of the
+// largest difference
+__device__ __forceinline__ uint32_t rel_first(const double *f, const int (&nd)[8], double (&d)[8])
 {
   const double f0 = f[nd[0]];
+  uint32_t top = 0;
+  d[0] = 0.;
+#pragma unroll
+  for (int k = 1; k < 8; k++) {
+    d[k] = RSUB(f[nd[k]], f0);
+    top = max(top, f64_mag(d[k]));
+  }
+  return top;
+}
+// The transform of such differences times 2^k (k20 = k << 20).  The sign product of the directions in m
+// at node b is (-1)^|m| (-1)^popcount(m & b).
+__device__ __forceinline__ void walsh_of(const double (&d)[8], int k20, ff (&w)[8])
+{
   float b = 0.f;
   w[0] = ff{0.f, 0.f};
 #pragma unroll
   for (int k = 1; k < 8; k++) {
-    const double d = RSUB(f[nd[k]], f0);
-    top = max(top, f64_mag(d));
-    w[sign_place(k)] = ff_of(d);
+    w[sign_place(k)] = ff_of(d[k], k20);
     b = f_max(b, f_abs(w[sign_place(k)].h));
   }
   const float C = grid_of(8.f * b);
@@ -308,7 +319,9 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
 #pragma unroll
     for (int r = 0; r < DIM; r++) {
       ff w[NEN];
-      walsh_rel(a.x[r], nd, top, w);
+      double d[NEN];
+      top = max(top, rel_first(a.x[r], nd, d));
+      walsh_of(d, 0, w);
       hg.x[0][r] = w[3];
       hg.x[1][r] = w[6];
       hg.x[2][r] = w[5];
@@ -318,7 +331,8 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         J[r][c] = ff_scale(ff_neg(w[1 << c]), 0.125f);
         mJ[c] = f_max(mJ[c], f_abs(J[r][c].h));
       }
-      walsh_rel(a.du[r], nd, top, w);
+      top = max(top, rel_first(a.du[r], nd, d));
+      walsh_of(d, 0, w);
 #pragma unroll
       for (int c = 0; c < DIM; c++) {
         GU[r][c] = ff_scale(ff_neg(w[1 << c]), 0.125f);
@@ -326,6 +340,20 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     }
   }
   bool bad = !mf.ok || !c_tolFF.ok || top >= (uint32_t)((1023 + 60) << 20);
+  if constexpr (ET == DNL_ELHEX8N3D_1PT) {
+    // the hourglass forces' factors: speeds below 2^39 (infinities and NaN are above it), rho c and the
+    // coefficient within ranges whose product a float holds.  The state is stored before the forces are
+    // formed, so this is looked at here.
+    uint32_t topV = 0;
+#pragma unroll
+    for (int k = 0; k < NEN; k++) {
+      const int n = __ldg(a.conn + (long)k * a.E + e);
+#pragma unroll
+      for (int r = 0; r < DIM; r++) topV = max(topV, f64_mag(a.v[r][n]));
+    }
+    const uint32_t c = f64_mag(a.hourglass), lo = (uint32_t)((1023 - 20) << 20);
+    bad |= topV >= (uint32_t)((1023 + 39) << 20) || !mf.okHg || (c != 0u && c - lo >= (uint32_t)(40 << 20));
+  }
 
   // ---- scaled by a power of two to entries below 1 (exact; G_u with it, so that G is unchanged)
   float mj = mJ[0];
@@ -785,11 +813,13 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     for (int k = 0; k < 8; k++) nd[k] = __ldg(a.conn + (long)k * a.E + e);
     const float sc = bits_f((uint32_t)(127 - js) << 23);
     ff q[4][3], gv[3][3];
-    uint32_t topV = 0;
+    int jv[3];  // velocities' component r is over 2^jv[r]
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       ff w[8];
-      walsh_rel(a.v[r], nd, topV, w);
+      double d[8];
+      jv[r] = (int)(rel_first(a.v[r], nd, d) >> 20) - 1023;
+      walsh_of(d, -jv[r] * (1 << 20), w);
       q[0][r] = w[3];
       q[1][r] = w[6];
       q[2][r] = w[5];
@@ -827,10 +857,16 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     // a_h = coefficient rho c V^(2/3) / 4 over 2^k, V = 8 detJ; the volume's sign does not matter
     // (an element that is turned inside out or numbered the other way round is no error in 3D)
     const ff vol = ff_scale(det.h < 0.f ? ff_neg(det) : det, 8.f);
-    const ff ah = ff_mul(ff_mul(mf.rhoCs4, ff_of(a.hourglass)), pow23_ff(vol));
+    const ff ah0 = ff_mul(ff_mul(mf.rhoCs4, ff_of(a.hourglass)), pow23_ff(vol));
 #pragma unroll
     for (int r = 0; r < 3; r++) {
+      // M and the hourglass part are added over 2^ef, the larger one's power of two, so that either alone
+      // keeps its precision however small it is against 2^k
       ff P[3], F[8];
+      const float mM = f_max(f_abs(M[0][r].h), f_max(f_abs(M[1][r].h), f_abs(M[2][r].h)));
+      const int ef = max((int)(f_bits(mM) >> 23) - 127, jv[r]);
+      const float sM = bits_f((uint32_t)(127 - ef) << 23), sv = jv[r] - ef < -100 ? 0.f : bits_f((uint32_t)(127 + jv[r] - ef) << 23);
+      const ff ah = ff_scale(ah0, sv);
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         ff t = ff_mul(hg.x[0][i], q[0][r]);
@@ -845,7 +881,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         ff t = ff_mul(Ji[l][0], P[0]);
         t = ff_add(t, ff_mul(Ji[l][1], P[1]));
         t = ff_add(t, ff_mul(Ji[l][2], P[2]));
-        F[1 << l] = ff_neg(ff_sub(M[l][r], ff_scale(ff_mul(ah, t), 0.125f)));
+        F[1 << l] = ff_neg(ff_sub(ff_scale(M[l][r], sM), ff_scale(ff_mul(ah, t), 0.125f)));
       }
       F[3] = ff_mul(ah, q[0][r]);
       F[6] = ff_mul(ah, q[1][r]);
@@ -863,7 +899,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
       walsh8(F);
       if (put) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) a.fe[(long)r * a.feStride + (long)e * NEN + k] = f64_of(ff_neg(ff_norm(F[sign_place(k)].h, F[sign_place(k)].l)), f20);
+        for (int k = 0; k < 8; k++) a.fe[(long)r * a.feStride + (long)e * NEN + k] = f64_of(ff_neg(ff_norm(F[sign_place(k)].h, F[sign_place(k)].l)), f20 + ef * (1 << 20));
       }
     }
   }

@@ -823,6 +823,7 @@ struct MatFF {
   float c4, c5, c6, c7, c8;
   float n3;                      // what the pair n leaves of the exponent
   ff rhoCs4;                     // rho c / 4 over 2^k (the one-point hexahedron's hourglass viscosity)
+  int okHg;                      // rho c is 0 or within 2^-40 .. 2^40 of 2^k
 };
 
 inline MatFF make_mat_ff(double G2, double G3, double K, double A, double B, double n, double dfun0,
@@ -852,6 +853,7 @@ inline MatFF make_mat_ff(double G2, double G3, double K, double A, double B, dou
   m.c7 = (float)((n - 6.) / 7.);
   m.c8 = (float)((n - 7.) / 8.);
   m.rhoCs4 = ff_host(0.25 * rhoCs * s);
+  m.okHg = rhoCs == 0. || (rhoCs * s >= 0x1p-40 && rhoCs * s <= 0x1p40);
   return m;
 }
 

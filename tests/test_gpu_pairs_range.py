@@ -16,6 +16,8 @@ TOL = 1e-12
 
 def rel(a, b):
     a, b = np.asarray(a).ravel(), np.asarray(b).ravel()
+    top = max(np.abs(b).max(initial=0.0), 1e-300)  # squares of large values overflow
+    a, b = a / top, b / top
     return np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
 
 
@@ -38,4 +40,36 @@ def test_inverted_one_point_hexahedra(gpu_lib, hourglass):
     m.conn = m.conn.copy()
     m.conn[::2] = m.conn[::2][:, [4, 5, 6, 7, 0, 1, 2, 3]]
     want, got, _, _ = both(gpu_lib, m, states.random_state(m, seed=21, du_scale=1e-4))
+    assert rel(got, want) <= TOL
+
+
+@pytest.mark.parametrize("speed", [float("nan"), float("inf"), -1e300, 1e40, 1e-30])
+def test_hourglass_velocities_of_any_size(gpu_lib, speed):
+    """One node's speed out of the pairs' range, or all tiny: the other nodes' forces are not touched, and
+    infinities and NaN come out where the oracle has them."""
+    m = meshes.taylor_hex_1pt(5, 3)
+    st = states.random_state(m, seed=22, du_scale=1e-4)
+    if abs(speed) < 1.0:
+        st["v"] *= speed
+        st["S"][...] = st["p"][...] = st["du"][...] = 0.0  # hourglass forces alone
+    else:
+        st["v"][7, 1] = speed
+    want, got, _, _ = both(gpu_lib, m, st)
+    want, got = want.reshape(m.N, 3), got.reshape(m.N, 3)
+    near = np.zeros(m.N, dtype=bool)
+    near[np.unique(m.conn[(m.conn == 7).any(axis=1)])] = True
+    assert np.array_equal(np.isfinite(want), np.isfinite(got))
+    assert rel(got[~near], want[~near]) <= TOL
+    for c in range(3):
+        ok = np.isfinite(want[near, c])
+        assert rel(got[near, c][ok], want[near, c][ok]) <= TOL
+
+
+@pytest.mark.parametrize("coefficient,density", [(1e-9, 8930.0), (1.0, 8930.0), (0.05, 1e-24), (0.05, 1e30)])
+def test_hourglass_factors_of_any_size(gpu_lib, coefficient, density):
+    m = meshes.taylor_hex_1pt(5, 3)
+    m.hourglass, m.density = coefficient, density
+    st = states.random_state(m, seed=23, du_scale=1e-4)
+    st["S"][...] = st["p"][...] = st["du"][...] = 0.0
+    want, got, _, _ = both(gpu_lib, m, st)
     assert rel(got, want) <= TOL
