@@ -197,48 +197,66 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
   float2 *const sh = reinterpret_cast<float2 *>(red);  // this element's shared memory
   const ff zero = {0.f, 0.f};
 
-  // ---- J and G_u from differences of nodal values: FP64 differences, pairs from there on
+  // ---- J and G_u from differences of nodal values: FP64 differences, pairs from there on.  Lengths are
+  // over 2^js, the power of two above the element's largest coordinate difference: one scale for the
+  // element, as its lanes exchange products of their J, and taken before the conversion, so that the
+  // unit of length does not matter (exact, and G is unchanged).
   ff J[DIM][DIM], GU[DIM][DIM];
   ff Rad = zero, vR = zero;
-  uint32_t top = 0;  // largest high word of the differences
+  uint32_t top = 0, topX = 0;  // largest high words: of the lane's other lengths, of the differences of x
+  int js;
   float mJ[DIM];
   HourglassX hg;  // the one-point hexahedron's
+  auto scale_of = [&]() {
+#pragma unroll
+    for (int o = 1; o < NIP; o <<= 1) topX = max(topX, __shfl_xor_sync(0xffffffffu, topX, o));
+    js = (int)(topX >> 20) - 1022;
+    return -js * (1 << 20);
+  };
   if constexpr (EDGES) {
     using EG = Edges<ET>;
     constexpr int NE = EG::NE, PER = NE / DIM;
     float2 *ex = sh, *eu = sh + NE * DIM;
+    double dx[DIM], du[DIM], dh[DIM];  // the lane's edge, and half of another
     {
       const int lo = __ldg(a.conn + (long)edge_node(EG::LO, pt) * a.E + e);
       const int hi = __ldg(a.conn + (long)edge_node(EG::HI, pt) * a.E + e);
 #pragma unroll
       for (int r = 0; r < DIM; r++) {
-        const double dx = RSUB(a.x[r][hi], a.x[r][lo]), du = RSUB(a.du[r][hi], a.du[r][lo]);
-        top = max(top, max(f64_mag(dx), f64_mag(du)));
-        ex[pt * DIM + r] = f2(ff_of(dx));
-        eu[pt * DIM + r] = f2(ff_of(du));
+        dx[r] = RSUB(a.x[r][hi], a.x[r][lo]);
+        du[r] = RSUB(a.du[r][hi], a.du[r][lo]);
+        topX = max(topX, f64_mag(dx[r]));
+        top = max(top, f64_mag(du[r]));
       }
     }
+    const int eg2 = NIP + (pt & (NIP / 2 - 1));
+    const bool isx = pt < NIP / 2;
     if constexpr (NE > NIP) {  // the hexahedron's other four edges: x on one half of the lanes, u on the other
       static_assert(NE == NIP + NIP / 2, "edges per lane");
-      const int eg = NIP + (pt & (NIP / 2 - 1));
-      const bool isx = pt < NIP / 2;
-      const int lo = __ldg(a.conn + (long)edge_node(EG::LO, eg) * a.E + e);
-      const int hi = __ldg(a.conn + (long)edge_node(EG::HI, eg) * a.E + e);
-      float2 *const to = isx ? ex : eu;
+      const int lo = __ldg(a.conn + (long)edge_node(EG::LO, eg2) * a.E + e);
+      const int hi = __ldg(a.conn + (long)edge_node(EG::HI, eg2) * a.E + e);
 #pragma unroll
       for (int r = 0; r < DIM; r++) {
         const double *src = isx ? a.x[r] : a.du[r];
-        const double d = RSUB(src[hi], src[lo]);
-        top = max(top, f64_mag(d));
-        to[eg * DIM + r] = f2(ff_of(d));
+        dh[r] = RSUB(src[hi], src[lo]);
+        const uint32_t t = f64_mag(dh[r]);
+        topX = max(topX, isx ? t : 0u);
+        top = max(top, isx ? 0u : t);
       }
+    }
+    const int j20 = scale_of();
+#pragma unroll
+    for (int r = 0; r < DIM; r++) {
+      ex[pt * DIM + r] = f2(ff_of(dx[r], j20));
+      eu[pt * DIM + r] = f2(ff_of(du[r], j20));
+      if constexpr (NE > NIP) (isx ? ex : eu)[eg2 * DIM + r] = f2(ff_of(dh[r], j20));
     }
     if (AXI) {  // the nodes' radii and radial displacements
       const int nd = __ldg(a.conn + (long)pt * a.E + e);
       const double x0 = a.x[0][nd], u0 = a.du[0][nd];
       top = max(top, max(f64_mag(x0), f64_mag(u0)));
-      sh[2 * NE * DIM + pt] = f2(ff_of(x0));
-      sh[2 * NE * DIM + NEN + pt] = f2(ff_of(u0));
+      sh[2 * NE * DIM + pt] = f2(ff_of(x0, j20));
+      sh[2 * NE * DIM + NEN + pt] = f2(ff_of(u0, j20));
     }
     __syncwarp();
 #pragma unroll
@@ -293,17 +311,26 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     __syncwarp();  // the force assembly reuses the buffer
   } else if constexpr (ET == DNL_ELTET4N3D) {
     int nd[4];
+    double dx[3][3], du[3][3];  // [component][axis]
 #pragma unroll
     for (int k = 0; k < 4; k++) nd[k] = __ldg(a.conn + (long)k * a.E + e);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        dx[r][c] = RSUB(a.x[r][nd[c + 1]], a.x[r][nd[0]]);
+        du[r][c] = RSUB(a.du[r][nd[c + 1]], a.du[r][nd[0]]);
+        topX = max(topX, f64_mag(dx[r][c]));
+        top = max(top, f64_mag(du[r][c]));
+      }
+    const int j20 = scale_of();
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       mJ[c] = 0.f;
 #pragma unroll
       for (int r = 0; r < 3; r++) {
-        const double dx = RSUB(a.x[r][nd[c + 1]], a.x[r][nd[0]]), du = RSUB(a.du[r][nd[c + 1]], a.du[r][nd[0]]);
-        top = max(top, max(f64_mag(dx), f64_mag(du)));
-        J[r][c] = ff_of(dx);
-        GU[r][c] = ff_of(du);
+        J[r][c] = ff_of(dx[r][c], j20);
+        GU[r][c] = ff_of(du[r][c], j20);
         mJ[c] = f_max(mJ[c], f_abs(J[r][c].h));
       }
     }
@@ -312,16 +339,19 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     // node signs in pairs: J and G_u (1/8 of the linear coefficients), the hourglass coefficients of
     // x, all coefficients of v
     int nd[NEN];
+    double dx[DIM][NEN];
 #pragma unroll
     for (int k = 0; k < NEN; k++) nd[k] = __ldg(a.conn + (long)k * a.E + e);
+#pragma unroll
+    for (int r = 0; r < DIM; r++) topX = max(topX, rel_first(a.x[r], nd, dx[r]));
+    const int j20 = scale_of();
 #pragma unroll
     for (int c = 0; c < DIM; c++) mJ[c] = 0.f;
 #pragma unroll
     for (int r = 0; r < DIM; r++) {
       ff w[NEN];
       double d[NEN];
-      top = max(top, rel_first(a.x[r], nd, d));
-      walsh_of(d, 0, w);
+      walsh_of(dx[r], j20, w);
       hg.x[0][r] = w[3];
       hg.x[1][r] = w[6];
       hg.x[2][r] = w[5];
@@ -332,14 +362,16 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         mJ[c] = f_max(mJ[c], f_abs(J[r][c].h));
       }
       top = max(top, rel_first(a.du[r], nd, d));
-      walsh_of(d, 0, w);
+      walsh_of(d, j20, w);
 #pragma unroll
       for (int c = 0; c < DIM; c++) {
         GU[r][c] = ff_scale(ff_neg(w[1 << c]), 0.125f);
       }
     }
   }
-  bool bad = !mf.ok || !c_tolFF.ok || top >= (uint32_t)((1023 + 60) << 20);
+  // lengths within 2^-200 .. 2^200, none above 2^60 of the element's size (what is below 2^-70 of it is 0;
+  // of displacements that is less than FP64 resolves in F)
+  bool bad = !mf.ok || !c_tolFF.ok || js < -200 || js > 200 || (int)top >= (1022 + 60 + js) << 20;
   if constexpr (ET == DNL_ELHEX8N3D_1PT) {
     // the hourglass forces' factors: speeds below 2^39 (infinities and NaN are above it), rho c and the
     // coefficient within ranges whose product a float holds.  The state is stored before the forces are
@@ -355,27 +387,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     bad |= topV >= (uint32_t)((1023 + 39) << 20) || !mf.okHg || (c != 0u && c - lo >= (uint32_t)(40 << 20));
   }
 
-  // ---- scaled by a power of two to entries below 1 (exact; G_u with it, so that G is unchanged)
-  float mj = mJ[0];
-#pragma unroll
-  for (int c = 1; c < DIM; c++) mj = f_max(mj, mJ[c]);
-  // one scale for the element: its lanes exchange products of their J
-#pragma unroll
-  for (int o = 1; o < NIP; o <<= 1) mj = f_max(mj, __shfl_xor_sync(0xffffffffu, mj, o));
-  const int js = (int)(f_bits(mj) >> 23) - 126;  // mj < 2^js
-  bad |= !(mj > 0x1p-60f);
-  {
-    const float sc = bits_f((uint32_t)(127 - js) << 23);
-#pragma unroll
-    for (int c = 0; c < DIM; c++) {
-      mJ[c] *= sc;
-#pragma unroll
-      for (int r = 0; r < DIM; r++) {
-        J[r][c] = ff_scale(J[r][c], sc);
-        GU[r][c] = ff_scale(GU[r][c], sc);
-      }
-    }
-  }
   // ---- adjugate, determinant, G = G_u J^-1
   ff adj[DIM][DIM], det, rdet, G[3][3];
   bad |= !deform_ff<DIM>(J, GU, mJ, adj, det, rdet, G);
@@ -420,7 +431,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         tape(TL::GU + l * DIM + c, f64_of(GU[l][c], j20));
       }
     tape(TL::DETJ, f64_of(det, DIM * j20));
-    tape(TL::RAD, AXI ? f64_of(Rad) : 0.);
+    tape(TL::RAD, AXI ? f64_of(Rad, j20) : 0.);
     tape(TL::VRR, AXI ? f64_of(G[2][2]) : 0.);
 #pragma unroll
     for (int k = 0; k < 9; k++) {
@@ -727,10 +738,9 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     for (int l = 0; l < DIM; l++)
 #pragma unroll
       for (int i = 0; i < DIM; i++) M[l][i] = ff_mul(M[l][i], twoPiR);
-    // sigma_tt / R x W, W = detJ 2 pi R; in the scale of M (detJ has one factor 2^js more)
-    hoop = ff_scale(ff_mul(ff_mul(Sn[2], det), FF_CONST(kDeuxPi)), bits_f((uint32_t)(127 + js) << 23));
+    hoop = ff_mul(ff_mul(Sn[2], det), FF_CONST(kDeuxPi));  // sigma_tt / R x W, W = detJ 2 pi R
   }
-  const int f20 = k20 + (DIM - 1) * js * (1 << 20);  // forces' exponent: stress x length^(DIM-1)
+  const int f20 = k20 + (DIM - 1 + (AXI ? 1 : 0)) * js * (1 << 20);  // forces' exponent: stress x length^(DIM-1)
   if constexpr (NEN == NIP) {
     // Node k's force is sum_q sum_l dN_k,l(q) M_q[l] (+ N_k(q) hoop_q).  With s_b(k) the sign of node
     // k's (and Gauss point k's) coordinate b and g = 1/sqrt(3), dN_k,l(q) = s_l(k) / 2^DIM prod_(b != l)
@@ -811,7 +821,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     int nd[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) nd[k] = __ldg(a.conn + (long)k * a.E + e);
-    const float sc = bits_f((uint32_t)(127 - js) << 23);
     ff q[4][3], gv[3][3];
     int jv[3];  // velocities' component r is over 2^jv[r]
 #pragma unroll
@@ -833,10 +842,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     for (int l = 0; l < 3; l++)
 #pragma unroll
       for (int c = 0; c < 3; c++) Ji[l][c] = ff_mul(adj[l][c], rdet);
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) hg.x[k][i] = ff_scale(hg.x[k][i], sc);
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       ff g[3];

@@ -73,3 +73,26 @@ def test_hourglass_factors_of_any_size(gpu_lib, coefficient, density):
     st["S"][...] = st["p"][...] = st["du"][...] = 0.0
     want, got, _, _ = both(gpu_lib, m, st)
     assert rel(got, want) <= TOL
+
+
+MODELS = {"axi": lambda: meshes.taylor_axi(5, 7), "plane": lambda: meshes.taylor_plane(3, 9),
+          "hex": lambda: meshes.taylor_hex(5, 3), "tet4": lambda: meshes.taylor_tet(3, 3),
+          "hex1pt": lambda: meshes.taylor_hex_1pt(5, 3)}
+
+
+@pytest.mark.parametrize("unit", [1e-40, 1e-16, 1e-12, 1e-9, 1e9, 1e40])
+@pytest.mark.parametrize("name", sorted(MODELS))
+def test_any_unit_of_length(gpu_lib, name, unit):
+    """Increments of 1e-6 of an edge (stresses of 1e5 beside 1e8) in small and large units of length."""
+    m = MODELS[name]()
+    st = states.random_state(m, seed=24, du_scale=1e-6)
+    st["v"][...] = 0.0
+    m.coords = m.coords * unit
+    st["coords"], st["du"] = st["coords"] * unit, st["du"] * unit
+    want, got, o, d = both(gpu_lib, m, st)
+    assert rel(got / unit, want / unit) <= TOL
+    for k, v in d.get_state("S", "Eps", "EpsPlas", "p", "evp").items():
+        assert rel(v, o.array(k)) <= TOL, k
+    # the increment itself, not only the state that it is added to
+    dS = (d.get_state("p")["p"].ravel() - st["p"].ravel())
+    assert rel(dS, o.array("p").ravel() - st["p"].ravel()) <= 1e-9
