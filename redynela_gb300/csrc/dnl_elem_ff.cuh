@@ -498,6 +498,12 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     }
     topS = max(topS, f64_mag(pd));
     bad |= topS >= (uint32_t)(((1023 + 50) << 20) + k20);
+    // Eps and EpsPlas are read further down, when parts of the element may be stored: their high words here
+    uint32_t topE = 0;
+#pragma unroll
+    for (int k = 0; k < NS; k++)
+      topE = max(topE, max(f64_mag_at(a.ip + (Ly::EPS + k) * nIP + ipx), f64_mag_at(a.ip + (Ly::EPSP + k) * nIP + ipx)));
+    bad |= topE >= (uint32_t)((1023 + 100) << 20);
     const ff tr3 = ff_mul(trace, FF_CONST(1. / 3.));
 #pragma unroll
     for (int k = 0; k < NS; k++) {
@@ -532,7 +538,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
       const ff one = {1.f, 0.f};
       ff evF = zero, Bx = zero, revp = zero, Sig0, h0;
       if (power) {
-        bad |= f64_mag(evpn) >= (uint32_t)((1023 + 60) << 20);
+        bad |= f64_mag(evpn) >= (uint32_t)((1023 + 30) << 20);
         evF = ff_of(evp);
         Bx = ff_mul(mf.B, ff_of(evpn));
         revp = ff_rcp(evF);
@@ -586,6 +592,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
             break;
           }
         }
+        bad |= !(f_abs(gamma.h) < 0x1p30f);  // no root: a table whose slope cancels 3 G
         gi = ff_mul(gamma, inv);
         const double xv = f64_add(evp, ff_mul(FF_CONST(kSqrt23), gamma));
         if (TAPE) {
@@ -692,7 +699,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
 #pragma unroll
       for (int k = 0; k < NS; k++) {
         in[k] = t > 0 || plastic ? ff_from(hold[(t * NS + k) * HOLD]) : zero;
-        Sn[k] = ff_add(ff_of_any(Xd[k], -kt), in[k]);
+        Sn[k] = ff_add(ff_of(Xd[k], -kt), in[k]);
       }
       rfi_ff<TWO_D>(Q, mq, Sn, D);
 #pragma unroll

@@ -212,17 +212,11 @@ FFD ff ff_of(double x, int k20 = 0)
   r.l = ok ? m * ulp52 : 0.f;
   return r;
 }
-// the same with NaN for |x| >= 2^100, infinities and NaN
-FFD ff ff_of_any(double x, int k20 = 0)
-{
-  ff r = ff_of(x, k20);
-  if ((uint32_t)(d_bits(x) >> 32 & 0x7fffffffu) >= (uint32_t)((1023 + 100) << 20)) r.h = bits_f(0x7fc00000u);
-  return r;
-}
 // (h + l) 2^k as a double for a normalised pair, rounded to nearest, without an FP64 instruction: the
 // high part's bits, and the low part as a whole number of the high part's FP64 ulps added to them as
 // a 64-bit integer.  Where h is a power of two and l takes the sum below it an ulp is half as large.
-// |h| below 2^-75 is converted without l, 0 and subnormal h give 0.
+// |h| below 2^-75 is converted without l, 0 and subnormal h give 0.  For finite pairs: an infinite or
+// NaN h would come out as a number near 2^128, so the element pass looks at its inputs' ranges first.
 FFD double f64_of(ff a, int k20 = 0)
 {
   const uint32_t b = f_bits(a.h), sign = b & 0x80000000u;
@@ -243,6 +237,7 @@ FFD double f64_of(ff a, int k20 = 0)
 FFD double f64_add(double x, ff a, int k20 = 0) { return x + f64_of(a, k20); }
 // high word of |x| (orders like |x|): for range checks without FP64 compares
 FFD uint32_t f64_mag(double x) { return (uint32_t)(d_bits(x) >> 32) & 0x7fffffffu; }
+FFD uint32_t f64_mag_at(const double *x) { return reinterpret_cast<const uint32_t *>(x)[1] & 0x7fffffffu; }  // that word alone
 
 // ------------------------------------------------------------------------ grid accumulation
 // C = 1.5 2^k with 2^(k-1) the power of two at or above bound (finite, >= 0)
@@ -830,7 +825,8 @@ inline MatFF make_mat_ff(double G2, double G3, double K, double A, double B, dou
                          double rhoCs)
 {
   MatFF m;
-  auto in_range = [G2](double x) { return x == 0. || (fabs(x) < 0x1p60 * G2 && fabs(x) > 0x1p-60 * G2); };
+  // with evp^n below 2^30 and its growth below 2^58 the products stay below 2^120
+  auto in_range = [G2](double x) { return x == 0. || (fabs(x) < 0x1p30 * G2 && fabs(x) > 0x1p-60 * G2); };
   m.ok = G2 > 0x1p-400 && G2 < 0x1p400 && in_range(G3) && in_range(K) && in_range(A) && in_range(B) && fabs(n) < 64.;
   int k = 0;
   frexp(m.ok ? G2 : 1., &k);

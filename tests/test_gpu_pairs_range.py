@@ -96,3 +96,49 @@ def test_any_unit_of_length(gpu_lib, name, unit):
     # the increment itself, not only the state that it is added to
     dS = (d.get_state("p")["p"].ravel() - st["p"].ravel())
     assert rel(dS, o.array("p").ravel() - st["p"].ravel()) <= 1e-9
+
+
+# (a finite stress of that size has no return mapping: an error status)
+@pytest.mark.parametrize("field,value", [(f, v) for f in ("S", "Eps", "EpsPlas", "p") for v in (float("nan"), float("inf"), 1e35, -1e200)
+                                         if f != "S" or not np.isfinite(v)])
+@pytest.mark.parametrize("name", sorted(MODELS))
+def test_state_out_of_range(gpu_lib, name, field, value):
+    """One point's component out of the pairs' range: infinities and NaN stay that, numbers are the
+    oracle's, and no other element is touched.  (Which other components an infinity reaches depends on
+    the zeros that a form leaves out and on its yield test, so they are not compared.)"""
+    m = MODELS[name]()
+    st = states.random_state(m, seed=25, du_scale=1e-4)
+    st["v"][...] = 0.0
+    st[field].reshape(m.E * m.nip, -1)[5, 0] = value
+    want, got, o, d = both(gpu_lib, m, st)
+    own = np.arange(m.E) == 5 // m.nip
+    for k, v in d.get_state("S", "Eps", "EpsPlas", "p", "evp").items():
+        g, w = v.reshape(m.E, m.nip, -1), o.array(k).reshape(m.E, m.nip, -1)
+        rest = np.full(m.E, True) if np.isfinite(value) and k != field else ~own
+        assert rel(g[rest], w[rest]) <= TOL, k
+        if k == field:
+            if np.isfinite(w[own]).all():
+                assert rel(g[own], w[own]) <= TOL, k
+            assert np.isfinite(g[own][0, 5 % m.nip, 0]) == np.isfinite(w[own][0, 5 % m.nip, 0])
+    nodes = np.ones(m.N, dtype=bool)
+    nodes[m.conn[own]] = False
+    g, w = got.reshape(m.N, m.dim), want.reshape(m.N, m.dim)
+    assert rel(g[nodes], w[nodes]) <= TOL
+    if field in ("S", "p"):
+        assert np.array_equal(np.isfinite(g[~nodes]).all(axis=1), np.isfinite(w[~nodes]).all(axis=1))
+
+
+@pytest.mark.parametrize("unit", [1e-60, 1e-20, 1e20, 1e60])
+@pytest.mark.parametrize("name", sorted(MODELS))
+def test_any_unit_of_stress(gpu_lib, name, unit):
+    m = MODELS[name]()
+    st = states.random_state(m, seed=26, du_scale=1e-4)
+    for k in ("young", "A", "B"):
+        setattr(m, k, getattr(m, k) * unit)
+    m.density *= unit  # the hourglass viscosity with it
+    st["S"], st["p"] = st["S"] * unit, st["p"] * unit
+    want, got, o, d = both(gpu_lib, m, st)
+    assert rel(got / unit, want / unit) <= TOL
+    for k, v in d.get_state("S", "Eps", "EpsPlas", "p", "evp").items():
+        u = unit if k in ("S", "p") else 1.0
+        assert rel(v / u, o.array(k) / u) <= TOL, k
