@@ -641,9 +641,13 @@ FFD bool strain_ff(const ff (&G)[3][3], ff (&E)[6], float mg, ff tol, int cap, i
     ff S2[6];
     mul_sym<TWO_D>(E, E, C2, S2);
     // remainders of ln(1 + x)/2 and (1 + x)^(-1/2) per eigenvalue, to matrices through V: from x^3 on
-    // (level 0, |E'| <= 2^-10), x^5 (level 1, 2^-6) or x^8 (level 2)
+    // (level 0, |x| <= 2^-10), x^5 (level 1, 2^-6) or x^8 (level 2).  The lines lie where the remainder's
+    // rounding in single precision (2^-24 of x^3/6, x^5/10) is 2^-56 at most.  By the eigenvalues: they reach
+    // three times the entries, and with the entries' size the error was 9e-17 at |G| = 2^-11 and 6e-16
+    // at 2^-7 (root mean square of ln U, FP64 6e-17), now 8e-18 and 5e-17.
     const float ev[3] = {f00.h + f00.l, f11.h + f11.l, f22.h + f22.l};
-    const int level = me <= 0x1p-10f ? 0 : (me <= 0x1p-6f ? 1 : 2);
+    const float mv = f_max(f_abs(ev[0]), f_max(f_abs(ev[1]), f_abs(ev[2])));
+    const int level = mv <= 0x1p-10f ? 0 : (mv <= 0x1p-6f ? 1 : 2);
     float gl[3], gh[3];
 #pragma unroll
     for (int m = 0; m < 3; m++) {
