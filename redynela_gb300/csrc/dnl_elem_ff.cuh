@@ -262,7 +262,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
 #pragma unroll
     for (int c = 0; c < DIM; c++) {
       ff w[PER], dx[PER][DIM], du[PER][DIM];
-      float bu = 0.f;
 #pragma unroll
       for (int q = 0; q < PER; q++) {
         const int eg = c * PER + q;
@@ -271,23 +270,21 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         for (int r = 0; r < DIM; r++) {
           dx[q][r] = ff_from(ex[eg * DIM + r]);
           du[q][r] = ff_from(eu[eg * DIM + r]);
-          bu = f_max(bu, f_abs(du[q][r].h));
         }
       }
-      // the weights of an axis sum to 1/2 (the table's signs are those of the + end)
-      const float CU = grid_of(0.50001f * bu);
       mJ[c] = 0.f;
 #pragma unroll
       for (int r = 0; r < DIM; r++) {
-        Dot sx(dx[0][r], w[0]);
-        Acc su(CU);
+        // both sums compensated: G_u on a grid of its edges' size cost ln U more than all that follows
+        // (hexahedra, |G| = 2^-7: 1.1e-16 against 4.0e-17, FP64 5.6e-17)
+        Dot sx(dx[0][r], w[0]), su(du[0][r], w[0]);
 #pragma unroll
-        for (int q = 0; q < PER; q++) {
-          if (q) sx.mac(dx[q][r], w[q]);
+        for (int q = 1; q < PER; q++) {
+          sx.mac(dx[q][r], w[q]);
           su.mac(du[q][r], w[q]);
         }
         J[r][c] = sx.get();
-        GU[r][c] = su.get(CU);
+        GU[r][c] = su.get();
         mJ[c] = f_max(mJ[c], f_abs(J[r][c].h));
       }
     }

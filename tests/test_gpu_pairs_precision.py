@@ -1,0 +1,129 @@
+"""How precise the element pass's kinematics and polar decomposition are: ln U and R of single elements
+against extended precision, for increments on both sides of every line between the pairs' forms and the FP64
+form.
+
+Bounds (root mean square over points and components): rounding F = I + G to FP64 costs its diagonal up to
+2^-53, and ln U as much; R = F U^-1 is a sum of products of rounded factors near 1, four times that."""
+
+import numpy as np
+import pytest
+
+from redynela_gb300 import meshes
+
+pytestmark = pytest.mark.gpu
+LD = np.longdouble
+ETYPES = {"axi": meshes.ELQUA4NAX, "plane": meshes.ELQUA4N2D, "hex": meshes.ELHEX8N3D, "tet4": meshes.ELTET4N3D,
+          "hex1pt": meshes.ELHEX8N3D_1PT}
+QUAD = np.array([[0, 0], [1, 0], [1, 1], [0, 1]], float)
+HEX = np.array([[*xy, z] for z in (0, 1) for xy in QUAD], float)
+TET = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
+
+
+def _nodes(et):
+    return QUAD if et in (meshes.ELQUA4NAX, meshes.ELQUA4N2D) else TET if et == meshes.ELTET4N3D else HEX
+
+
+def _tables(et):
+    """Shape values (q, k) and derivatives (q, k, c) at the integration points, extended precision."""
+    if et == meshes.ELTET4N3D:
+        return np.full((1, 4), LD(1) / 4), np.array([[[-1, -1, -1], [1, 0, 0], [0, 1, 0], [0, 0, 1]]], LD)
+    sign = 2 * _nodes(et).astype(LD) - 1
+    pts = np.zeros((1, 3), LD) if et == meshes.ELHEX8N3D_1PT else sign / np.sqrt(LD(3))
+    f = 1 + pts[:, None, :] * sign[None]
+    d = sign.shape[1]
+    D = np.stack([sign[None, :, c] * np.prod(np.delete(f, c, axis=2), axis=2) for c in range(d)], axis=2) / LD(2) ** d
+    return np.prod(f, axis=2) / LD(2) ** d, D
+
+
+def _inverse(J):
+    d = J.shape[-1]
+    A = np.empty_like(J)
+    if d == 2:
+        A[..., 0, 0], A[..., 0, 1], A[..., 1, 0], A[..., 1, 1] = J[..., 1, 1], -J[..., 0, 1], -J[..., 1, 0], J[..., 0, 0]
+    else:
+        for r in range(3):
+            for c in range(3):
+                u, v, p, q = (c + 1) % 3, (c + 2) % 3, (r + 1) % 3, (r + 2) % 3
+                A[..., r, c] = J[..., u, p] * J[..., v, q] - J[..., v, p] * J[..., u, q]
+    return A / sum(J[..., 0, c] * A[..., c, 0] for c in range(d))[..., None, None]
+
+
+def _polar(G):
+    """ln U and R from G = F - I: the reference's pivots, rotations and stop at 1e-9, on C - I."""
+    n, I = len(G), np.arange(len(G))
+    one = np.eye(3, dtype=LD)
+    E, V = G + G.transpose(0, 2, 1) + np.einsum("nki,nkj->nij", G, G), np.tile(one, (n, 1, 1))
+    for _ in range(29):
+        q1 = np.abs(E[:, 0, 1]) > np.abs(E[:, 0, 2])
+        p0 = np.where(q1, np.abs(E[:, 0, 1]), np.abs(E[:, 0, 2])) > np.abs(E[:, 1, 2])
+        p, q = np.where(p0, 0, 1), np.where(p0 & q1, 1, 2)
+        x = E[I, p, q]
+        go = np.abs(x) >= LD("1e-9")
+        al = (E[I, q, q] - E[I, p, p]) / (2 * np.where(go, x, 1))
+        t = np.where(go, 1 / (np.abs(al) + np.sqrt(al * al + 1)) * np.where(al < 0, -1, 1), 0)
+        R = np.tile(one, (n, 1, 1))
+        R[I, p, p] = R[I, q, q] = 1 / np.sqrt(1 + t * t)
+        R[I, p, q], R[I, q, p] = t * R[I, p, p], -t * R[I, p, p]
+        E, V = np.einsum("nji,njk,nkl->nil", R, E, R), np.einsum("nij,njk->nik", V, R)
+    lam = np.einsum("nii->ni", E)
+    F = G + one
+    return np.einsum("nik,nk,njk->nij", V, np.log1p(lam) / 2, V), F @ np.einsum("nik,nk,njk->nij", V, 1 / np.sqrt(1 + lam), V)
+
+
+def _elements(et, size, seed, shear=0.0):
+    """Separate distorted elements at some distance from the origin, displaced by gradients whose largest
+    entry is `size` (a third each random, nearly rank one, simple shear), with a little noise."""
+    rng = np.random.default_rng(seed)
+    ref = _nodes(et)
+    dim, E, h = ref.shape[1], 48, 1e-3
+    X = ref[None] * h + rng.uniform(-0.1, 0.1, (E,) + ref.shape) * h
+    X = X @ (np.eye(dim) + shear * np.triu(np.ones((dim, dim)), 1)).T
+    off = rng.uniform(5.0, 60.0, (E, 1, dim)) * h
+    G = rng.normal(size=(E, dim, dim))
+    a = rng.choice([-1.0, 1.0], size=(E, dim))
+    G[::3] = (a[:, :, None] * a[:, None, :] * (1 + 0.02 * rng.uniform(-1, 1, G.shape)))[::3]
+    G[1::3] = 0.02 * G[1::3]
+    G[1::3, 0, dim - 1] = 1.0
+    G *= (size / np.abs(G).max(axis=(1, 2)))[:, None, None]
+    u = np.einsum("eij,ekj->eki", G, X - X.mean(axis=1, keepdims=True)) + rng.normal(scale=1e-3 * size * h, size=X.shape)
+    X = X + off
+    N = E * len(ref)
+    x3, u3 = np.zeros((N, 3)), np.zeros((N, 3))
+    x3[:, :dim], u3[:, :dim] = X.reshape(N, dim), u.reshape(N, dim)
+    m = meshes.Model(et, x3, np.arange(N).reshape(E, -1), tend=1.0,
+                     method=meshes.PULSE if et == meshes.ELHEX8N3D else meshes.COURANT)
+    return m, x3, u3
+
+
+def _reference(et, x3, u3):
+    k = len(_nodes(et))
+    dim = _nodes(et).shape[1]
+    N, D = _tables(et)
+    x, u = (a.reshape(-1, k, 3)[..., :dim].astype(LD) for a in (x3, u3))
+    Ji = _inverse(np.einsum("ekr,qkc->eqrc", x, D))
+    G = np.zeros(Ji.shape[:2] + (3, 3), LD)
+    G[..., :dim, :dim] = np.einsum("ekr,qkl,eqlc->eqrc", u, D, Ji)
+    if et == meshes.ELQUA4NAX:
+        G[..., 2, 2] = np.einsum("qk,ek->eq", N, u[..., 0]) / np.einsum("qk,ek->eq", N, x[..., 0])
+    return _polar(G.reshape(-1, 3, 3))
+
+
+def _rms(a):
+    return float(np.sqrt(np.mean(np.square(a.astype(LD)))))
+
+
+def check(gpu_lib, name, size, seed, shear=0.0):
+    et = ETYPES[name]
+    m, x3, u3 = _elements(et, size, seed, shear)
+    d = gpu_lib.GpuDomain(m, gpu_lib.FLAG_STEP_TENSORS)
+    d.internal_forces(x3, u3)
+    lnU, R = (a.reshape(-1, 3, 3) for a in d.step_tensors())
+    want = _reference(et, x3, u3)
+    assert _rms(lnU - want[0]) <= 2.0 ** -53
+    assert _rms(R - want[1]) <= 2.0 ** -51
+
+
+@pytest.mark.parametrize("exponent", [-7, -8, -9, -10, -11.1, -12.6, -16, -30])
+@pytest.mark.parametrize("name", ["axi", "hex", "plane", "tet4"])
+def test_increments(gpu_lib, name, exponent):
+    check(gpu_lib, name, 2.0 ** exponent, 40)
