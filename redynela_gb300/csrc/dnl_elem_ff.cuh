@@ -60,18 +60,23 @@ __device__ __forceinline__ ff axN_ff(int pt, int k)
   return d == 0 ? c_shapeFF.axN[0] : (d == 1 ? c_shapeFF.axN[1] : c_shapeFF.axN[2]);
 }
 
-// Walsh transform of eight values on one grid: after it, entry m is sum_b (-1)^popcount(m & b) v_b.
-// Sums and differences of such pairs are exact in the high parts (the grid's bound covers the sums).
+// Walsh transform of eight values, the first of them 0: after it, entry m is sum_b (-1)^popcount(m & b) v_b.
+// Sums and differences with their rounding errors: on one grid for all eight values, two additions each
+// instead of eight, the low parts lost 2^-44 of the largest value, and with them J and G_u
+// (ln U at |G| = 2^-8: 1.6e-16 root mean square, now 1.8e-17, FP64 5.8e-17) and the hourglass forces (1.5e-13
+// of themselves, now 8e-15; FP64 3e-14 at 5 to 60 edges from the origin, where its sums round).
 __device__ __forceinline__ void walsh8(ff (&v)[8])
 {
+  v[0] = v[1];
+  v[1] = ff_neg(v[1]);
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-    for (int b = 0; b < 8; b++)
+    for (int b = o == 1 ? 2 : 0; b < 8; b++)
       if (!(b & o)) {
         const ff p = v[b], q = v[b | o];
-        v[b] = ff{p.h + q.h, p.l + q.l};
-        v[b | o] = ff{p.h - q.h, p.l - q.l};
+        v[b] = ff_add_raw(p, q);
+        v[b | o] = ff_add_raw(p, ff_neg(q));
       }
 }
 // node k's place: bit 0, 1, 2 set where xi, eta, zeta = +1
@@ -94,20 +99,8 @@ __device__ __forceinline__ uint32_t rel_first(const double *f, const int (&nd)[8
 // at node b is (-1)^|m| (-1)^popcount(m & b).
 __device__ __forceinline__ void walsh_of(const double (&d)[8], int k20, ff (&w)[8])
 {
-  float b = 0.f;
-  w[0] = ff{0.f, 0.f};
 #pragma unroll
-  for (int k = 1; k < 8; k++) {
-    w[sign_place(k)] = ff_of(d[k], k20);
-    b = f_max(b, f_abs(w[sign_place(k)].h));
-  }
-  const float C = grid_of(8.f * b);
-#pragma unroll
-  for (int k = 1; k < 8; k++) {
-    Acc s(C);
-    s.add(w[k]);
-    w[k] = s.raw(C);
-  }
+  for (int k = 1; k < 8; k++) w[sign_place(k)] = ff_of(d[k], k20);
   walsh8(w);
 #pragma unroll
   for (int k = 1; k < 8; k++) w[k] = ff_norm(w[k].h, w[k].l);
@@ -117,15 +110,17 @@ struct HourglassX {
   ff x[4][3];
 };
 // x^(2/3) of a positive pair within the float range: seed by the hardware exponential and logarithm
-// base 2, one Newton step of y^3 = x with the residual in pairs
+// base 2, two Newton steps of y^3 = x with the residual in pairs (one left 1e-13, the rounding of its
+// correction of 1e-6)
 __device__ __forceinline__ ff pow23_ff(ff x)
 {
-  const float y0 = exp2f(log2f(x.h) * (1.f / 3.f));
-  const ff y = {y0, 0.f};
-  const ff y2 = ff_mul(y, y), r = ff_sub(x, ff_mul(y2, y));
-  const float d = r.h / (3.f * y2.h);        // first-order correction ...
-  const ff c = ff_norm(y0, d - d * d / y0);  // ... and the second-order one
-  return ff_mul(c, c);
+  ff y = {exp2f(log2f(x.h) * (1.f / 3.f)), 0.f};
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const ff y2 = ff_mul(y, y), r = ff_sub(x, ff_mul(y2, y));
+    y = ff_norm(y.h, y.l + r.h * (f_rcp(y2.h) * (1.f / 3.f)));
+  }
+  return ff_mul(y, y);
 }
 
 // The first pivot of the polar decomposition (0: C01, 1: C02, 2: C12) from C in FP64 with the
@@ -883,8 +878,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
         for (int k = 1; k < 4; k++) t = ff_add(t, ff_mul(hg.x[k][i], q[k][r]));
         P[i] = t;
       }
-      float mF = 0.f;
-      F[0] = zero;
 #pragma unroll
       for (int l = 0; l < 3; l++) {
         ff t = ff_mul(Ji[l][0], P[0]);
@@ -896,15 +889,6 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
       F[6] = ff_mul(ah, q[1][r]);
       F[5] = ff_mul(ah, q[2][r]);
       F[7] = ff_neg(ff_mul(ah, q[3][r]));
-#pragma unroll
-      for (int k = 1; k < 8; k++) mF = f_max(mF, f_abs(F[k].h));
-      const float C = grid_of(8.f * mF);
-#pragma unroll
-      for (int k = 1; k < 8; k++) {
-        Acc s(C);
-        s.add(F[k]);
-        F[k] = s.raw(C);
-      }
       walsh8(F);
       if (put) {
 #pragma unroll

@@ -124,6 +124,30 @@ def check(gpu_lib, name, size, seed, shear=0.0):
 
 
 @pytest.mark.parametrize("exponent", [-7, -8, -9, -10, -11.1, -12.6, -16, -30])
-@pytest.mark.parametrize("name", ["axi", "hex", "plane", "tet4"])
+@pytest.mark.parametrize("name", sorted(ETYPES))
 def test_increments(gpu_lib, name, exponent):
     check(gpu_lib, name, 2.0 ** exponent, 40)
+
+
+def test_hourglass_forces(gpu_lib):
+    """Hourglass forces alone, no stress and no increment.  Bound: the coefficient's and the projected
+    velocities' chains of some twenty pair operations of 2^-47, root mean square."""
+    et = meshes.ELHEX8N3D_1PT
+    m, x3, u3 = _elements(et, 2.0 ** -10, 41)
+    v = np.random.default_rng(41).normal(scale=50.0, size=x3.shape)
+    d = gpu_lib.GpuDomain(m)
+    d.set_state(v=v)
+    got = d.internal_forces(x3, 0.0 * u3).reshape(-1, 8, 3)
+    x, v = (a.reshape(-1, 8, 3).astype(LD) for a in (x3, v))
+    sign = 2 * HEX.astype(LD) - 1
+    D = _tables(et)[1][0]
+    J = np.einsum("ekr,kc->erc", x, D)
+    b = np.einsum("kl,elc->ekc", D, _inverse(J))
+    V = 8 * np.einsum("ei,ei->e", np.cross(J[:, :, 0], J[:, :, 1]), J[:, :, 2])
+    h = np.stack([sign[:, 0] * sign[:, 1], sign[:, 1] * sign[:, 2], sign[:, 2] * sign[:, 0], sign.prod(axis=1)])
+    g = h - np.einsum("qk,ekr,ejr->eqj", h, x, b)
+    young, nu, rho = LD(m.young), LD(m.poisson), LD(m.density)
+    c = np.sqrt(young * (1 - nu) / (rho * (1 + nu) * (1 - 2 * nu)))
+    ah = LD(m.hourglass) * rho * c * np.cbrt(V) ** 2 / 4
+    want = -ah[:, None, None] * np.einsum("eqk,eqr->ekr", g, np.einsum("eqk,ekr->eqr", g, v))
+    assert _rms(got - want) <= np.sqrt(20.0) * 2.0 ** -47 * _rms(want)
