@@ -172,7 +172,7 @@ constexpr int HOLD = 32;
 template <int ET> __host__ __device__ constexpr int hold_slots() { return 3 * Elem<ET>::NS; }
 
 // One Gauss point in pairs.  Returns true when its element needs the FP64 pass instead (an increment
-// above kFastMax, a badly shaped element, state or constants outside the pairs' range): then
+// above its limit, a badly shaped element, state or constants outside the pairs' range): then
 // nothing of the element is stored or recorded.  Uniform over the element's lanes; depends on the
 // element's own data only, so a warp's other elements do not matter.
 template <int ET, bool TAPE, bool GENERAL>
@@ -381,7 +381,9 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
 
   // ---- adjugate, determinant, G = G_u J^-1
   ff adj[DIM][DIM], det, rdet, G[3][3];
-  bad |= !deform_ff<DIM>(J, GU, mJ, adj, det, rdet, G);
+  float cols;
+  deform_ff<DIM>(J, GU, mJ, adj, det, rdet, G, cols);
+  bad |= !(f_abs(det.h) >= (TWO_D ? 0x1p-5f : 0x1p-6f) * cols);
   float mg = 0.f;
 #pragma unroll
   for (int r = 0; r < DIM; r++)
@@ -392,7 +394,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
     mg = f_max(mg, f_abs(G[2][2].h));
     bad |= !(Rad.h > 0x1p-60f);
   }
-  bad |= !(mg <= (TWO_D ? kFastMax2D : kFastMax));
+  bad |= !(mg <= kFastMax) || mg * cols > kShapeMax * kFastMax * f_abs(det.h);
 
   // ---- ln U and R - I
   ff E[6];

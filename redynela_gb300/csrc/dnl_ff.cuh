@@ -6,19 +6,18 @@
 // 6 FP32 instructions in the form below, ten times less, and the FP64 pipe stays free for what
 // needs it: coordinate differences and the sums into the stored FP64 state.
 //
-// Why it is precise enough: in an explicit step the strain increment is small (|F - I| <= 2^-6 for
-// the solids, kFastMax; larger increments take the FP64 path), and the pairs carry F - I, C - I, ln U and R - I
-// themselves, not 1 + them.  FP64 rounds 1 + x at 2^-53 absolute; a pair rounds x at 2^-47 relative.
-// Against 113-bit arithmetic from J and G_u on, random elements (root mean square error of ln U | R):
-// increments of 2^-6 1.7e-16 | 1.3e-16 here, 1.2e-16 | 5.0e-16 in FP64; 2^-8 3.6e-17 | 2.8e-17,
-// 1.1e-16 | 4.9e-16; from 2^-12 down 1.4e-17 | 1.5e-17, 1.1e-16 | 4.7e-16.  A whole force pass against
-// extended precision (jittered bars, mid-impact and random states): nodal forces 2 to 11 times, S 3 to
-// 11 times closer than the FP64 pass, every other field closer or as close.  The plane and
-// axisymmetric elements go to 2^-3 (kFastMax2D), which first-row elements reach in the first steps of
-// an impact; 200 steps of the 5 x 50 bar from the impact on end with S 4 to 5 times and v and p twice
-// closer to extended precision than with FP64, evp within 10 %.  A single pass there is the other way
-// round: at increments of 8e-2 S carries 5.7e-14 of its norm where FP64 has 5e-15; the two cross near
-// 2^-6.
+// Why it is precise enough: in an explicit step the strain increment is small (|F - I| <= kFastMax, 0.5 %;
+// larger increments take the FP64 path), and the pairs carry F - I, C - I, ln U and R - I themselves, not 1 +
+// them.  FP64 rounds 1 + x at 2^-53 absolute; a pair rounds x at 2^-47 relative.  Root mean square errors
+// of a force pass against 80-bit arithmetic, separate distorted elements at 5 to 60 edges from the origin,
+// six kinds of increments, hexahedra, pairs | FP64, stresses and forces relative:
+//   |G|      ln U               R                  S                  evp                forces
+//   2^-8     1.9e-17 | 5.5e-17  2.4e-17 | 2.0e-16  1.5e-14 | 4.0e-14  1.4e-16 | 1.9e-16  1.3e-14 | 4.6e-14
+//   2^-10    9e-18   | 5.5e-17  2.1e-17 | 2.0e-16  1.2e-14 | 6.0e-14  4.1e-17 | 1.2e-16  1.2e-14 | 6.9e-14
+//   2^-14.5  7e-18   | 5.7e-17  2.3e-17 | 1.8e-16  9e-15   | 7.1e-14  1.8e-17 | 4.8e-17  1.3e-14 | 1.0e-13
+// The other element types are alike.  Above the limit the stress, which the return maps back from a trial
+// value several times as large, and the plastic multiplier would carry more than FP64 (uniaxial increments
+// of 2^-7 in the quads: S 2.1 to 2.3 times FP64's error; evp of hexahedra 3.0e-16 | 2.0e-16).
 //
 // Error-free steps used: Knuth's two-sum, Dekker's fast two-sum, the product error by fma.  Dot
 // products accumulate on a fixed grid (Acc): the running sum starts at C = 1.5 2^k with 2^(k-1) an
@@ -344,21 +343,19 @@ FFD ff rsqrt1p_ff(ff x)
 }
 
 // ------------------------------------------------------------------------ kinematics
-// G = G_u J^-1 by the adjugate: adj(J) and det(J) too; mJ: largest entry of each column of J.
-// Returns false for a badly shaped element (|det J| small against its columns), whose differences
-// of products would cancel.
+// G = G_u J^-1 by the adjugate: adj(J) and det(J) too; mJ: largest entry of each column of J, cols: their
+// product, against which a badly shaped element's |det J| is small: its differences of products cancel.
 template <int DIM>
-FFD bool deform_ff(const ff (&J)[DIM][DIM], const ff (&GU)[DIM][DIM], const float (&mJ)[DIM],
-                   ff (&adj)[DIM][DIM], ff &det, ff &rdet, ff (&G)[3][3])
+FFD void deform_ff(const ff (&J)[DIM][DIM], const ff (&GU)[DIM][DIM], const float (&mJ)[DIM],
+                   ff (&adj)[DIM][DIM], ff &det, ff &rdet, ff (&G)[3][3], float &cols)
 {
-  bool good;
   if constexpr (DIM == 2) {
     adj[0][0] = J[1][1];
     adj[0][1] = ff_neg(J[0][1]);
     adj[1][0] = ff_neg(J[1][0]);
     adj[1][1] = J[0][0];
     det = ff_sub(ff_mul(J[0][0], J[1][1]), ff_mul(J[0][1], J[1][0]));
-    good = f_abs(det.h) >= 0x1p-5f * mJ[0] * mJ[1];
+    cols = mJ[0] * mJ[1];
   } else {
 #pragma unroll
     for (int l = 0; l < 3; l++) {
@@ -373,7 +370,7 @@ FFD bool deform_ff(const ff (&J)[DIM][DIM], const ff (&GU)[DIM][DIM], const floa
 #pragma unroll
     for (int r = 1; r < 3; r++) s.mac(J[r][0], adj[0][r]);
     det = s.get();
-    good = f_abs(det.h) >= 0x1p-6f * mJ[0] * mJ[1] * mJ[2];
+    cols = mJ[0] * mJ[1] * mJ[2];
   }
   rdet = ff_rcp(det);
 #pragma unroll
@@ -389,14 +386,17 @@ FFD bool deform_ff(const ff (&J)[DIM][DIM], const ff (&GU)[DIM][DIM], const floa
       for (int l = 1; l < DIM; l++) s.mac(GU[r][l], adj[l][c]);
       G[r][c] = ff_mul(s.get(), rdet);
     }
-  return good;
 }
 
 // ------------------------------------------------------------------------ polar decomposition
-// limit of |F - I|'s entries for the pair arithmetic
-constexpr float kFastMax = 0x1p-6f;    // solids
-constexpr float kFastMax2D = 0x1p-3f;  // plane and axisymmetric
-constexpr float kSeriesG = 0x1p-6f;    // limit of the power series
+// Limit of |F - I|'s entries for the pair arithmetic (2^-7.75): the errors of S and evp, the first to cross
+// FP64's, are the same there (uniaxial increments, pairs over FP64: S 0.8 (solids) to 1.4 (plane) at 2^-7.5,
+// 1.3 to 2.3 at 2^-7; evp of all kinds of increments 0.7 to 0.9 at 2^-8, 1.0 to 1.2 at 2^-7.5).  For distorted elements
+// G = G_u J^-1 carries the pairs' error times the products' cancellation, so the limit falls with the ratio
+// of the product of J's columns to det J: from kShapeMax on, a hexahedron with columns sheared by 2 crosses
+// FP64 at 2^-8.2, by 3 at 2^-9.0, by 4 at 2^-9.7, its ratio being 1.2, 2.3 and 3.9 times kShapeMax.
+constexpr float kFastMax = 0x1.3p-8f;
+constexpr float kShapeMax = 1.8f;
 
 // symmetric component order of the six-entry arrays: xx yy zz xy xz yz
 FFD constexpr int sym_i(int k) { return k < 3 ? k : (k == 5 ? 1 : 0); }
@@ -512,7 +512,6 @@ FFD bool strain_ff(const ff (&G)[3][3], ff (&E)[6], float mg, ff tol, int cap, i
       for (int j = 0; j < 3; j++) Vk[i][j] = ff{i == j ? 1.f : 0.f, 0.f};
   }
   bool conv = false, rotated = false;
-  ff c2d = {1.f, 0.f}, s2d = {0.f, 0.f};  // plane case: the one rotation
   for (int it = 1; it <= cap; it++) {
     // pivot of Tensor2.C:1173-1178: q = |C01| > |C02| ? 1 : 2, p = |C0q| > |C12| ? 0 : 1
     int k = 0;
@@ -556,8 +555,6 @@ FFD bool strain_ff(const ff (&G)[3][3], ff (&E)[6], float mg, ff tol, int cap, i
         f00 = a2;
         f11 = b2;
         f01 = zero;
-        c2d = c;
-        s2d = s;
       } else {
         const ff y = k == 0 ? f02 : f01, z = k == 2 ? f02 : f12;
         Acc u(C), v(C);
@@ -601,146 +598,129 @@ FFD bool strain_ff(const ff (&G)[3][3], ff (&E)[6], float mg, ff tol, int cap, i
     lam[2] = ff_norm(f22.h, f22.l);
   }
   ff H[6];
-  float me;
-  if (TWO_D && mg > kSeriesG) {
-    // the plane case's larger increments: the functions of the eigenvalues themselves, rotated back
-    const ff x[3] = {ff_norm(f00.h, f00.l), ff_norm(f11.h, f11.l), ff_norm(f22.h, f22.l)};
-    const ff cc = ff_mul(c2d, c2d), ss = ff_mul(s2d, s2d), cs = ff_mul(c2d, s2d);
-    auto back = [&](ff a0, ff a1, ff a2, ff (&M)[6]) {
-      M[0] = ff_add(ff_mul(cc, a0), ff_mul(ss, a1));
-      M[1] = ff_add(ff_mul(ss, a0), ff_mul(cc, a1));
-      M[2] = a2;
-      M[3] = ff_mul(cs, ff_sub(a1, a0));
-      M[4] = M[5] = ff{0.f, 0.f};
-    };
-    back(half_log1p_ff(x[0]), half_log1p_ff(x[1]), half_log1p_ff(x[2]), L);
-    back(rsqrt1p_ff(x[0]), rsqrt1p_ff(x[1]), rsqrt1p_ff(x[2]), H);
-    me = f_max(f_abs(x[0].h), f_max(f_abs(x[1].h), f_abs(x[2].h)));
-  } else {
-    // E' = E - V r V^T; without a rotation V = I and E' is E's diagonal
-    {
-      const float r01 = f01.h + f01.l, r02 = f02.h + f02.l, r12 = f12.h + f12.l;
+  // E' = E - V r V^T; without a rotation V = I and E' is E's diagonal
+  {
+    const float r01 = f01.h + f01.l, r02 = f02.h + f02.l, r12 = f12.h + f12.l;
 #pragma unroll
-      for (int k = 0; k < (TWO_D ? 4 : 6); k++) {
-        const int i = sym_i(k), j = sym_j(k);
-        float K = 0.f;
-        if (!TWO_D || k != 2) {
-          K = r01 * f_fma(V[i][0], V[j][1], V[i][1] * V[j][0]);
-          if (!TWO_D) {
-            K = f_fma(r02, f_fma(V[i][0], V[j][2], V[i][2] * V[j][0]), K);
-            K = f_fma(r12, f_fma(V[i][1], V[j][2], V[i][2] * V[j][1]), K);
-          }
+    for (int k = 0; k < (TWO_D ? 4 : 6); k++) {
+      const int i = sym_i(k), j = sym_j(k);
+      float K = 0.f;
+      if (!TWO_D || k != 2) {
+        K = r01 * f_fma(V[i][0], V[j][1], V[i][1] * V[j][0]);
+        if (!TWO_D) {
+          K = f_fma(r02, f_fma(V[i][0], V[j][2], V[i][2] * V[j][0]), K);
+          K = f_fma(r12, f_fma(V[i][1], V[j][2], V[i][2] * V[j][1]), K);
         }
-        const ff e = ff_norm(E[k].h, E[k].l - K);
-        E[k] = rotated || i == j ? e : ff{0.f, 0.f};
       }
+      const ff e = ff_norm(E[k].h, E[k].l - K);
+      E[k] = rotated || i == j ? e : ff{0.f, 0.f};
     }
-    me = max_sym<TWO_D>(E);
-    constexpr int DN = TWO_D ? 2 : 3;
-    const float C2 = grid_of(DN * me * me);
-    ff S2[6];
-    mul_sym<TWO_D>(E, E, C2, S2);
-    // remainders of ln(1 + x)/2 and (1 + x)^(-1/2) per eigenvalue, to matrices through V: from x^3 on
-    // (level 0, |x| <= 2^-10), x^5 (level 1, 2^-6) or x^8 (level 2).  The lines lie where the remainder's
-    // rounding in single precision (2^-24 of x^3/6, x^5/10) is 2^-56 at most.  By the eigenvalues: they reach
-    // three times the entries, and with the entries' size the error was 9e-17 at |G| = 2^-11 and 6e-16
-    // at 2^-7 (root mean square of ln U, FP64 6e-17), now 8e-18 and 5e-17.
-    const float ev[3] = {f00.h + f00.l, f11.h + f11.l, f22.h + f22.l};
-    const float mv = f_max(f_abs(ev[0]), f_max(f_abs(ev[1]), f_abs(ev[2])));
-    const int level = mv <= 0x1p-10f ? 0 : (mv <= 0x1p-6f ? 1 : 2);
-    float gl[3], gh[3];
+  }
+  const float me = max_sym<TWO_D>(E);
+  constexpr int DN = TWO_D ? 2 : 3;
+  const float C2 = grid_of(DN * me * me);
+  ff S2[6];
+  mul_sym<TWO_D>(E, E, C2, S2);
+  // remainders of ln(1 + x)/2 and (1 + x)^(-1/2) per eigenvalue, to matrices through V: from x^3 on
+  // (level 0, |x| <= 2^-10), x^5 (level 1, 2^-6) or x^8 (level 2).  The lines lie where the remainder's
+  // rounding in single precision (2^-24 of x^3/6, x^5/10) is 2^-56 at most.  By the eigenvalues: they reach
+  // three times the entries, and with the entries' size the error was 9e-17 at |G| = 2^-11 and 6e-16
+  // at 2^-7 (root mean square of ln U, FP64 6e-17), now 8e-18 and 5e-17.
+  const float ev[3] = {f00.h + f00.l, f11.h + f11.l, f22.h + f22.l};
+  const float mv = f_max(f_abs(ev[0]), f_max(f_abs(ev[1]), f_abs(ev[2])));
+  const int level = mv <= 0x1p-10f ? 0 : (mv <= 0x1p-6f ? 1 : 2);
+  float gl[3], gh[3];
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    const float x = ev[m], x3 = x * x * x;
+    float l, h;
+    if (level == 2) {  // to x^15; the next is below 2^-60
+      l = f_fma(x, f_fma(x, f_fma(x, 1.f / 30.f, -1.f / 28.f), 1.f / 26.f), -1.f / 24.f);
+      l = f_fma(x, f_fma(x, f_fma(x, f_fma(x, l, 1.f / 22.f), -1.f / 20.f), 1.f / 18.f), -1.f / 16.f);
+      h = f_fma(x, f_fma(x, f_fma(x, -0.14446444809436798f, 0.14944598078727722f), -0.15498101711273193f), 0.16118025779724121f);
+      h = f_fma(x, f_fma(x, f_fma(x, f_fma(x, h, -88179.f / 524288.f), 46189.f / 262144.f), -12155.f / 65536.f), 6435.f / 32768.f);
+      const float x8 = x3 * x3 * x * x;
+      gl[m] = x8 * l;
+      gh[m] = x8 * h;
+    } else {
+      l = f_fma(x, f_fma(x, f_fma(x, 1.f / 18.f, -1.f / 16.f), 1.f / 14.f), -1.f / 12.f);
+      h = f_fma(x, f_fma(x, f_fma(x, -12155.f / 65536.f, 6435.f / 32768.f), -429.f / 2048.f), 231.f / 1024.f);
+      l = f_fma(x, l, 0.1f);
+      h = f_fma(x, h, -63.f / 256.f);
+      gl[m] = x3 * (level == 0 ? f_fma(x, f_fma(x, l, -0.125f), 1.f / 6.f) : x * x * l);
+      gh[m] = x3 * (level == 0 ? f_fma(x, f_fma(x, h, 35.f / 128.f), -5.f / 16.f) : x * x * h);
+    }
+  }
+  // P, R: the parts of fourth and higher order (ln and inverse root) that are formed as pairs
+  ff S3[6], P[6], R[6];
+  if (level > 0) {
+    ff S4[6];
+    const float m4 = DN * DN * DN * me * me * me * me;
+    mul_sym<TWO_D>(E, S2, grid_of(DN * DN * me * me * me), S3);
+    mul_sym<TWO_D>(S2, S2, grid_of(m4), S4);
+    if (level == 1) {
+#pragma unroll
+      for (int k = 0; k < 6; k++) {
+        P[k] = ff_scale(S4[k], -0.125f);
+        R[k] = ff_mulf(S4[k], 35.f / 128.f);
+      }
+    } else {  // E'^4 (c4 + c5 E' + c6 E'^2 + c7 E'^3)
+      ff A[6], B[6];
+#pragma unroll
+      for (int k = 0; k < 6; k++) {
+        if (TWO_D && k > 3) {
+          A[k] = B[k] = ff{0.f, 0.f};
+          continue;
+        }
+        Acc a(1.5f), b(1.5f);
+        a.macf(E[k], 0.1f);
+        a.macf(S2[k], -1.f / 12.f);
+        a.macf(S3[k], 1.f / 14.f);
+        b.macf(E[k], -63.f / 256.f);
+        b.macf(S2[k], 231.f / 1024.f);
+        b.macf(S3[k], -429.f / 2048.f);
+        if (k < 3) {
+          a.add(ff{-0.125f, 0.f});
+          b.add(ff{35.f / 128.f, 0.f});
+        }
+        A[k] = a.get(1.5f);
+        B[k] = b.get(1.5f);
+      }
+      mul_sym<TWO_D>(S4, A, grid_of(0.5f * m4), P);
+      mul_sym<TWO_D>(S4, B, grid_of(m4), R);
+    }
+  }
+  // the first-order parts by sums of pairs, the rest on the grid of its own size
+  const float CL = grid_of(0.625f * DN * me * me);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const int i = sym_i(k), j = sym_j(k);
+    if (TWO_D && k > 3) {
+      L[k] = H[k] = ff{0.f, 0.f};
+      continue;
+    }
+    float rl = 0.f, rh = 0.f;
 #pragma unroll
     for (int m = 0; m < 3; m++) {
-      const float x = ev[m], x3 = x * x * x;
-      float l, h;
-      if (level == 2) {  // to x^15; the next is below 2^-60
-        l = f_fma(x, f_fma(x, f_fma(x, 1.f / 30.f, -1.f / 28.f), 1.f / 26.f), -1.f / 24.f);
-        l = f_fma(x, f_fma(x, f_fma(x, f_fma(x, l, 1.f / 22.f), -1.f / 20.f), 1.f / 18.f), -1.f / 16.f);
-        h = f_fma(x, f_fma(x, f_fma(x, -0.14446444809436798f, 0.14944598078727722f), -0.15498101711273193f), 0.16118025779724121f);
-        h = f_fma(x, f_fma(x, f_fma(x, f_fma(x, h, -88179.f / 524288.f), 46189.f / 262144.f), -12155.f / 65536.f), 6435.f / 32768.f);
-        const float x8 = x3 * x3 * x * x;
-        gl[m] = x8 * l;
-        gh[m] = x8 * h;
-      } else {
-        l = f_fma(x, f_fma(x, f_fma(x, 1.f / 18.f, -1.f / 16.f), 1.f / 14.f), -1.f / 12.f);
-        h = f_fma(x, f_fma(x, f_fma(x, -12155.f / 65536.f, 6435.f / 32768.f), -429.f / 2048.f), 231.f / 1024.f);
-        l = f_fma(x, l, 0.1f);
-        h = f_fma(x, h, -63.f / 256.f);
-        gl[m] = x3 * (level == 0 ? f_fma(x, f_fma(x, l, -0.125f), 1.f / 6.f) : x * x * l);
-        gh[m] = x3 * (level == 0 ? f_fma(x, f_fma(x, h, 35.f / 128.f), -5.f / 16.f) : x * x * h);
-      }
+      if (TWO_D && ((m == 2) != (i == 2))) continue;
+      const float vv = V[i][m] * V[j][m];
+      rl = f_fma(vv, gl[m], rl);
+      rh = f_fma(vv, gh[m], rh);
     }
-    // P, R: the parts of fourth and higher order (ln and inverse root) that are formed as pairs
-    ff S3[6], P[6], R[6];
+    Acc sl(CL), sh(CL);
+    sl.add(ff_scale(S2[k], -0.25f));
+    sh.macf(S2[k], 0.375f);
     if (level > 0) {
-      ff S4[6];
-      const float m4 = DN * DN * DN * me * me * me * me;
-      mul_sym<TWO_D>(E, S2, grid_of(DN * DN * me * me * me), S3);
-      mul_sym<TWO_D>(S2, S2, grid_of(m4), S4);
-      if (level == 1) {
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-          P[k] = ff_scale(S4[k], -0.125f);
-          R[k] = ff_mulf(S4[k], 35.f / 128.f);
-        }
-      } else {  // E'^4 (c4 + c5 E' + c6 E'^2 + c7 E'^3)
-        ff A[6], B[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-          if (TWO_D && k > 3) {
-            A[k] = B[k] = ff{0.f, 0.f};
-            continue;
-          }
-          Acc a(1.5f), b(1.5f);
-          a.macf(E[k], 0.1f);
-          a.macf(S2[k], -1.f / 12.f);
-          a.macf(S3[k], 1.f / 14.f);
-          b.macf(E[k], -63.f / 256.f);
-          b.macf(S2[k], 231.f / 1024.f);
-          b.macf(S3[k], -429.f / 2048.f);
-          if (k < 3) {
-            a.add(ff{-0.125f, 0.f});
-            b.add(ff{35.f / 128.f, 0.f});
-          }
-          A[k] = a.get(1.5f);
-          B[k] = b.get(1.5f);
-        }
-        mul_sym<TWO_D>(S4, A, grid_of(0.5f * m4), P);
-        mul_sym<TWO_D>(S4, B, grid_of(m4), R);
-      }
+      sl.mac(S3[k], ff{1.f / 6.f, (float)(1. / 6. - (double)(1.f / 6.f))});
+      sl.add(P[k]);
+      sh.macf(S3[k], -0.3125f);
+      sh.add(R[k]);
     }
-    // the first-order parts by sums of pairs, the rest on the grid of its own size
-    const float CL = grid_of(0.625f * DN * me * me);
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-      const int i = sym_i(k), j = sym_j(k);
-      if (TWO_D && k > 3) {
-        L[k] = H[k] = ff{0.f, 0.f};
-        continue;
-      }
-      float rl = 0.f, rh = 0.f;
-#pragma unroll
-      for (int m = 0; m < 3; m++) {
-        if (TWO_D && ((m == 2) != (i == 2))) continue;
-        const float vv = V[i][m] * V[j][m];
-        rl = f_fma(vv, gl[m], rl);
-        rh = f_fma(vv, gh[m], rh);
-      }
-      Acc sl(CL), sh(CL);
-      sl.add(ff_scale(S2[k], -0.25f));
-      sh.macf(S2[k], 0.375f);
-      if (level > 0) {
-        sl.mac(S3[k], ff{1.f / 6.f, (float)(1. / 6. - (double)(1.f / 6.f))});
-        sl.add(P[k]);
-        sh.macf(S3[k], -0.3125f);
-        sh.add(R[k]);
-      }
-      sl.addf(rl);
-      sh.addf(rh);
-      const ff e2 = ff_scale(E[k], 0.5f);
-      L[k] = ff_add(e2, sl.get(CL));
-      H[k] = ff_sub(sh.get(CL), e2);
-    }
+    sl.addf(rl);
+    sh.addf(rh);
+    const ff e2 = ff_scale(E[k], 0.5f);
+    L[k] = ff_add(e2, sl.get(CL));
+    H[k] = ff_sub(sh.get(CL), e2);
   }
   if (KEEP) {
 #pragma unroll

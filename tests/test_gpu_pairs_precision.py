@@ -5,6 +5,9 @@ form.
 Bounds (root mean square over points and components): rounding F = I + G to FP64 costs its diagonal up to
 2^-53, and ln U as much; R = F U^-1 is a sum of products of rounded factors near 1, four times that."""
 
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -14,6 +17,9 @@ pytestmark = pytest.mark.gpu
 LD = np.longdouble
 ETYPES = {"axi": meshes.ELQUA4NAX, "plane": meshes.ELQUA4N2D, "hex": meshes.ELHEX8N3D, "tet4": meshes.ELTET4N3D,
           "hex1pt": meshes.ELHEX8N3D_1PT}
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "redynela_gb300", "csrc")
+with open(os.path.join(CSRC, "dnl_ff.cuh")) as src:
+    LIMIT = float.fromhex(re.search(r"kFastMax = (\S+)f;", src.read()).group(1))  # |F - I| of the pairs' form
 QUAD = np.array([[0, 0], [1, 0], [1, 1], [0, 1]], float)
 HEX = np.array([[*xy, z] for z in (0, 1) for xy in QUAD], float)
 TET = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
@@ -72,7 +78,8 @@ def _polar(G):
 
 def _elements(et, size, seed, shear=0.0):
     """Separate distorted elements at some distance from the origin, displaced by gradients whose largest
-    entry is `size` (a third each random, nearly rank one, simple shear), with a little noise."""
+    entry is `size` (of each element, or of all; a third each random, nearly rank one, simple shear), with
+    a little noise."""
     rng = np.random.default_rng(seed)
     ref = _nodes(et)
     dim, E, h = ref.shape[1], 48, 1e-3
@@ -84,8 +91,9 @@ def _elements(et, size, seed, shear=0.0):
     G[::3] = (a[:, :, None] * a[:, None, :] * (1 + 0.02 * rng.uniform(-1, 1, G.shape)))[::3]
     G[1::3] = 0.02 * G[1::3]
     G[1::3, 0, dim - 1] = 1.0
-    G *= (size / np.abs(G).max(axis=(1, 2)))[:, None, None]
-    u = np.einsum("eij,ekj->eki", G, X - X.mean(axis=1, keepdims=True)) + rng.normal(scale=1e-3 * size * h, size=X.shape)
+    size = np.broadcast_to(size, E)[:, None, None]
+    G *= size / np.abs(G).max(axis=(1, 2), keepdims=True)
+    u = np.einsum("eij,ekj->eki", G, X - X.mean(axis=1, keepdims=True)) + 1e-3 * size * h * rng.normal(size=X.shape)
     X = X + off
     N = E * len(ref)
     x3, u3 = np.zeros((N, 3)), np.zeros((N, 3))
@@ -123,10 +131,26 @@ def check(gpu_lib, name, size, seed, shear=0.0):
     assert _rms(R - want[1]) <= 2.0 ** -51
 
 
-@pytest.mark.parametrize("exponent", [-7, -8, -9, -10, -11.1, -12.6, -16, -30])
-@pytest.mark.parametrize("name", sorted(ETYPES))
+# (the FP64 form of the one-point hexahedron sums absolute coordinates: 2^-53 up to 2^-5)
+@pytest.mark.parametrize("name,exponent", [(n, e) for n in sorted(ETYPES) for e in (-3, -4, -5, -6, -6.5, -7, -8, -9, -10, -11.1, -12.6, -16, -30)
+                                           if n != "hex1pt" or e <= -5])
 def test_increments(gpu_lib, name, exponent):
     check(gpu_lib, name, 2.0 ** exponent, 40)
+
+
+@pytest.mark.parametrize("shear", [1.0, 2.0])
+@pytest.mark.parametrize("exponent", [-6, -7.5, -8.1, -9, -12])
+@pytest.mark.parametrize("name", sorted(ETYPES))
+def test_increments_of_sheared_elements(gpu_lib, name, exponent, shear):
+    check(gpu_lib, name, 2.0 ** exponent, 42, shear)
+
+
+@pytest.mark.parametrize("near", [0.97, 1.03, "both"])
+@pytest.mark.parametrize("name", sorted(ETYPES))
+def test_increments_at_the_limit(gpu_lib, name, near):
+    """Below, above, and both in every warp."""
+    f = np.where(np.arange(48) % 3 == 1, 0.97, 1.03) if near == "both" else near
+    check(gpu_lib, name, LIMIT * f, 43)
 
 
 def test_hourglass_forces(gpu_lib):
