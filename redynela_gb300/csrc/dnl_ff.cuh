@@ -320,11 +320,14 @@ FFD ff atanh_series_ff(ff s)
   p = ff_add(ff_host(1. / 3.), ff_mul(u, p));
   return ff_add(one, ff_mul(u, p));
 }
-// ln(1 + x)/2 and (1 + x)^(-1/2) - 1 for |x| <= 0.4, each to 2^-46 of itself
+// ln(1 + x)/2 for -1/2 <= x <= 1, to 2^-45 of itself: ln r with r = sqrt(1 + x) from 1/sqrt 2 to sqrt 2, which is
+// 2 atanh(s), s = (r - 1)/(r + 1) = x / (1 + r)^2 within 0.172 (without the root s reaches 1/3, past the series)
 FFD ff half_log1p_ff(ff x)
 {
-  const ff s = ff_mul(x, ff_rcp(ff_add(ff{2.f, 0.f}, x)));
-  return ff_mul(s, atanh_series_ff(s));
+  const ff y = ff_add(ff{1.f, 0.f}, x);
+  const ff d = ff_add(ff{1.f, 0.f}, ff_sqrt(y, f_rsqrt(y.h)));
+  const ff s = ff_mul(x, ff_rcp(ff_mul(d, d)));
+  return ff_scale(ff_mul(s, atanh_series_ff(s)), 2.f);
 }
 // (ln(1 + a) - ln(1 + b)) / (2 (a - b)), 1 / (2 (1 + a)) in the limit, |a|, |b| <= 0.4: with w = 2 + a + b and
 // u = (a - b) / w it is atanh(u) / (u w), no difference of logarithms; where u is beyond the series the
@@ -336,6 +339,7 @@ FFD ff half_log_slope_ff(ff a, ff b)
   if (f_abs(u.h) <= 0.17f) return ff_mul(atanh_series_ff(u), rw);
   return ff_mul(ff_sub(half_log1p_ff(a), half_log1p_ff(b)), ff_rcp(d));
 }
+// (1 + x)^(-1/2) - 1 for -1/2 <= x <= 1, to 2^-45 of itself
 FFD ff rsqrt1p_ff(ff x)
 {
   const ff y = ff_add(ff{1.f, 0.f}, x);

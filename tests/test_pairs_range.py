@@ -1,6 +1,6 @@
 """The pair arithmetic of csrc/dnl_ff.cuh at the ends of the ranges that it is used in, compiled for the
 host and compared with extended precision: nearly rank-one displacement gradients, whose eigenvalues are
-three times their entries, at the lines between the lengths of the series.
+three times their entries, at the lines between the lengths of the series; the eigenvalues' functions.
 
 Bounds: those of the pair itself, 2^-44 of the increment for a few dozen operations, and three times
 2^-22 of the stop's 1e-9 (terms that the reference drops go through single precision)."""
@@ -45,6 +45,12 @@ template <bool TWO_D, bool KEEP> void polar_t(int n, const double *g, double *L,
   }
 }
 extern "C" {
+void functions(int n, const double *x, double *half_log, double *rsqrt) {
+  for (int i = 0; i < n; i++) {
+    half_log[i] = f64_of(half_log1p_ff(ff_host(x[i])));
+    rsqrt[i] = f64_of(rsqrt1p_ff(ff_host(x[i])));
+  }
+}
 void polar(int two, int keep, int n, const double *g, double *L, double *Q, double *H, double *rest) {
   if (two)
     keep ? polar_t<true, true>(n, g, L, Q, H, rest) : polar_t<true, false>(n, g, L, Q, H, rest);
@@ -120,3 +126,20 @@ def check_polar(pairs, G, two, size):
 def test_rank_one_increments(pairs, exponent, two):
     size = 2.0 ** exponent
     check_polar(pairs, rank_one(np.random.default_rng(30), 200, size, two), two, size)
+
+
+def test_functions_of_an_eigenvalue(pairs):
+    """ln(1 + x)/2 and (1 + x)^(-1/2) - 1 over their whole range, -1/2 to 1.  Bound: relative, 2^-45 as they
+    state (half a dozen pair operations of 2^-47 and the series' 2^-47)."""
+    x = np.concatenate([np.linspace(-0.5, 1.0, 3001), np.geomspace(1e-12, 0.5, 200), -np.geomspace(1e-12, 0.5, 200)])
+    x = x[x != 0]
+    hl, rs = np.empty_like(x), np.empty_like(x)
+    pairs.functions(len(x), _p(x), _p(hl), _p(rs))
+    # the pair of x holds 2^-48 of it
+    hi = x.astype(np.float32).astype(np.float64)
+    e = hi.astype(np.longdouble) + (x - hi).astype(np.float32)
+    want = np.log1p(e) / 2
+    assert np.abs((hl - want) / want).max() <= 2.0 ** -45
+    y = 1 + e
+    want = -e / (y + np.sqrt(y))
+    assert np.abs((rs - want) / want).max() <= 2.0 ** -45
