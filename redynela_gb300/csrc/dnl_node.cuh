@@ -187,6 +187,7 @@ static __device__ void step_tail(const StepTail &t, DevTime *tm)
   }
   last = __shfl_sync(0xffffffffu, last, 0);
   if (!last) return;
+  __syncwarp();  // lane 0's fences order memory for the other lanes through this (a shuffle orders none)
   if (threadIdx.x == 0) tm->arrived = 0u;
   if (t.count) {
     for (int i = threadIdx.x; i < t.count; i += 32) {
