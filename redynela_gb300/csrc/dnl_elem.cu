@@ -1367,10 +1367,11 @@ template <int KIND>
 __global__ void __launch_bounds__(256) k_courant(ElemArgs a, StepTail tail)
 {
   after_previous();
-  if (a.tm->done | a.tm->status) return;
+  // no return here: another block may set the status meanwhile, and every block arrives at the tail
+  const bool live = !(a.tm->done | a.tm->status);
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double len = 1e300;
-  if (e < a.E) {
+  if (live && e < a.E) {
     len = elem_length<KIND>(a, e);
     if (!(len > 0.)) {
       record_error(a.tm, DNL_ERR_DT, a.eBase + e);
@@ -1384,7 +1385,7 @@ __global__ void __launch_bounds__(256) k_courant(ElemArgs a, StepTail tail)
   __shared__ double wmin[8];
   if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = len;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (live && threadIdx.x == 0) {
     double b = wmin[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = fmin(b, wmin[w]);
     atomicMin(&a.tm->lenMinBits, (unsigned long long)__double_as_longlong(b));

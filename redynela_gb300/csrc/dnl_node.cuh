@@ -173,7 +173,8 @@ static __device__ void sched_update(DevTime *tm, const double *dts, int phase)
 // Called by every thread of every block of a kernel once its work is done: the block that arrives
 // last runs the step's time logic, for which every other block has read the time record and written
 // its part.  Saves a launch and the gap before it (about 3.5 us of a step) against a kernel of one
-// thread.  The arrival counter is back at 0 afterwards.  Warp 0 of each block must not have left.
+// thread.  The arrival counter is back at 0 afterwards, so every block must arrive, also where the run
+// is over or has failed (the time logic looks at that itself).  Warp 0 of each block must not have left.
 static __device__ void step_tail(const StepTail &t, DevTime *tm)
 {
   if (!t.mode && !t.sched) return;
