@@ -67,9 +67,11 @@ __global__ void __launch_bounds__(128) k_node(NodeArgs g)
   after_previous();
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   DevTime *tm = g.tm;
-  if (tm->done | tm->status) return;  // set by earlier kernels or by this one's last block: all blocks alike
+  // set by earlier kernels or by this one's last block: all blocks alike.  The time logic runs all the same:
+  // scheduled steps count also in a run that is over.
+  const bool live = !(tm->done | tm->status);
   const NodeDt k = node_dt_block(tm->timeStep, g.ch);
-  if (n < g.N) node_update<DIM>(g, n, blockIdx.y, g.ch, k);
+  if (live && n < g.N) node_update<DIM>(g, n, blockIdx.y, g.ch, k);
   step_tail(g.tail, tm);
 }
 

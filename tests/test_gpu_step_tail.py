@@ -1,5 +1,5 @@
 """The time logic in the last block of a step's last kernel: after an error that some blocks of the Courant
-kernel see and others do not."""
+kernel see and others do not, and in scheduled steps of a run that is over."""
 
 import dataclasses
 
@@ -37,3 +37,19 @@ def test_time_step_after_a_courant_error(gpu_lib):
     d.step(10)
     assert abs(d.time_step() / want - 1.0) <= 1e-12
     assert np.array_equal(d.get_state("coords")["coords"], squeezed)
+
+
+def test_scheduled_steps_of_a_finished_run(gpu_lib, tmp_path):
+    """A restart at the end time: its steps do nothing, and a schedule counts its steps all the same."""
+    m = meshes.taylor_axi(4, 12, tend=2e-7)
+    d = gpu_lib.GpuDomain(m, gpu_lib.FLAG_STEP_TENSORS)
+    d.run()
+    path = str(tmp_path / "end.res")
+    d.write_results(path)
+    end = d.get_state("coords")["coords"]
+    r = gpu_lib.GpuDomain(m, gpu_lib.FLAG_STEP_TENSORS)
+    r.read_results(path)
+    assert r.step(1) == 0
+    x = r.run_schedule(np.full(7, 1e-9))
+    assert np.array_equal(x, end)
+    assert r.time_info()["increment"] == 7
