@@ -19,7 +19,8 @@ struct ShapeFF {
 };
 __constant__ ShapeFF c_shapeFF;
 // the polar decomposition's stopping test as a pair, and whether the tolerances are within the pairs'
-// reach (2^-52 for the polar decomposition, 2^-44 for the radial return; else every point is FP64's)
+// reach (2^-52 to 2^-29 for the polar decomposition, whose dropped terms, up to the tolerance, go through
+// single precision: at 1e-5 ln U would carry 9e-14; 2^-44 for the radial return; else every point is FP64's)
 struct TolFF {
   ff polar;
   int ok;
@@ -918,6 +919,6 @@ static bool set_tolerances_ff(double polar, double radial)
 {
   TolFF t;
   t.polar = ff_host(polar);
-  t.ok = polar >= 0x1p-52 && radial >= 0x1p-44;
+  t.ok = polar >= 0x1p-52 && polar <= 0x1p-29 && radial >= 0x1p-44;
   return cudaMemcpyToSymbol(c_tolFF, &t, sizeof t) == cudaSuccess;
 }
