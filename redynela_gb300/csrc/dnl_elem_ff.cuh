@@ -145,7 +145,8 @@ __device__ __noinline__ int pivot_f64(const ElemArgs &a, int e, int pt, double *
 }
 
 // The tabular law (hardening_law) with its stress and slope over 2^k as pairs; false past the table's
-// end, on a vertical segment and outside the pairs' range (FP64 then).  The search compares the doubles' bits (x > 0).
+// end, on a vertical or nearly vertical segment (below 2^-60: a width below 2^-70 would be converted to 0) and
+// outside the pairs' range (FP64 then).  The search compares the doubles' bits (x > 0).
 __device__ __forceinline__ bool table_ff(const HardLaw &m, double x, int k20, ff &sig, ff &h)
 {
   const double *X = m.tab, *Y = m.tab + m.tabN;
@@ -161,7 +162,7 @@ __device__ __forceinline__ bool table_ff(const HardLaw &m, double x, int k20, ff
   if (lo >= m.tabN) return false;
   const double x0 = __ldg(X + lo - 1), y0 = __ldg(Y + lo - 1), x1 = __ldg(X + lo), y1 = __ldg(Y + lo);
   const uint32_t top = (uint32_t)((1023 + 50) << 20);
-  if (x1 == x0 || max(f64_mag(x0), f64_mag(x1)) >= top || max(f64_mag(y0), f64_mag(y1)) >= top + (uint32_t)k20) return false;
+  if (f64_mag(x1 - x0) < (uint32_t)((1023 - 60) << 20) || max(f64_mag(x0), f64_mag(x1)) >= top || max(f64_mag(y0), f64_mag(y1)) >= top + (uint32_t)k20) return false;
   h = ff_mul(ff_of(y1 - y0, -k20), ff_rcp(ff_of(x1 - x0)));
   sig = ff_add(ff_of(y0, -k20), ff_mul(ff_of(x - x0), h));
   return true;

@@ -142,3 +142,20 @@ def test_any_unit_of_stress(gpu_lib, name, unit):
     for k, v in d.get_state("S", "Eps", "EpsPlas", "p", "evp").items():
         u = unit if k in ("S", "p") else 1.0
         assert rel(v / u, o.array(k) / u) <= TOL, k
+
+
+def test_nearly_vertical_segment_of_a_table(gpu_lib):
+    """evp = 1e-10 on a segment of the hardening table 1e-22 wide: the points yield there."""
+    m = meshes.taylor_hex(5, 3)
+    x = np.array([0.0, 1e-10 - 5e-23, 1e-10 + 5e-23, 0.1, 1.0, 10.0])
+    assert np.all(np.diff(x) > 0)
+    y = np.array([90e6, 90e6, 90e6 + 1e3, 150e6, 250e6, 400e6])
+    m.materials = [meshes.MaterialLaw(m.young, m.poisson, m.density, meshes.HARD_TABULAR, (), x, y)]
+    m.elem_material = np.zeros(m.E, dtype=np.int64)
+    st = states.random_state(m, seed=27, du_scale=1e-3)
+    st["evp"][...] = 1e-10
+    want, got, o, d = both(gpu_lib, m, st)
+    assert (o.array("evp") > 1e-9).sum() > 100  # yielded
+    assert rel(got, want) <= TOL
+    for k, v in d.get_state("S", "EpsPlas", "p", "evp").items():
+        assert rel(v, o.array(k)) <= TOL, k
