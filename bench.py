@@ -1,5 +1,6 @@
 #!/usr/bin/env python3
-"""Element-updates/s of DynELA's explicit step on GB300 (libdnlgpu, FP64).
+"""Element-updates/s of DynELA's explicit step on GB300 (libdnlgpu: FP64 state; the element pass in pairs
+of FP32 numbers where that is no less precise than FP64).
 
 Workload (default): the 3D Taylor impact bar of ElHex8n3D -- a 40x40 cross-section grid clipped
 to the radius, 400 layers (505,600 elements, 539,345 nodes), copper J2 material
@@ -38,17 +39,18 @@ sys.path.insert(0, ROOT)
 
 from redynela_gb300 import meshes  # noqa: E402
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_elem<ElHex8n3D> launch per element,
-# measured by ncu on the 126,400-element bar's mid-run window (308.85 MB); scaled by the elements
-# of the workload
-ELEM_TRAFFIC_BYTES_PER_ELEMENT = 308.85e6 / 126400
-
-# Instructions of one k_elem<ElHex8n3D> launch (the pass in pairs of FP32 numbers), from ncu's
-# smsp__inst_executed.sum on the bar cut to 60 layers of elements (606,720 points, early in the impact):
-# warp instructions per warp of 32 points; and the FP64 pipe's share of its peak there
-HEX_WARP_INSTR_PER_WARP = 177184265 / 18960
-HEX_FP64_PIPE_FRAC = 0.108
-HEX_INSTR_SOURCE = "75,840 hexahedra (40 x 40 x 60 layers) after 26 steps of the impact, ncu"
+# One k_elem<ElHex8n3D> launch of the pass in pairs of FP32 numbers in the timed window of the bar cut to
+# 100 layers of elements (126,400 elements, 31,600 warps, t = 10 us, plastic impact end), from ncu:
+# dram__bytes_read.sum + dram__bytes_write.sum per element, smsp__inst_executed.sum per warp of 32 points
+# (the 400-layer bar has a smaller share of plastic points, so the issue fraction formed with it is an upper
+# bound there) and the FP64 pipe's share of its peak
+ELEM_TRAFFIC_BYTES_PER_ELEMENT = (180.76e6 + 137.80e6) / 126400
+HEX_WARP_INSTR_PER_WARP = 347404248 / 31600
+HEX_FP64_PIPE_FRAC = 0.096
+HEX_INSTR_SOURCE = "126,400 hexahedra (40 x 40 x 100 layers) in the timed window (t = 10 us), ncu"
+# what `dtype` f64 stands for: state, results and everything outside the element pass
+ARITHMETIC = ("FP64 state and results; element pass in pairs of FP32 numbers, errors at or below those of the FP64 "
+              "form, which takes increments above 2^-7.75 and values out of range")
 
 
 def workload(name: str, layers: int = 400):
@@ -347,7 +349,7 @@ def main_ours(args):
     ms_max = barrier_and_max(ms, world)
     value = aggregate_rate(model.E * done, ms * 1e-3, world)
 
-    # ---- roofline of the dominant kernel (k_elem): the FP64 pipe binds it, HBM is reported beside
+    # ---- roofline of the dominant kernel (k_elem): instruction issue binds it, HBM is reported beside
     elem_ms, elem_n = prof["elem"]
     launch_s = elem_ms / elem_n * 1e-3 if elem_n else None
     roofline = issue_roofline(model, launch_s, clocks, local)
@@ -401,7 +403,7 @@ def main_ours(args):
                 "config": hex_config(model, name, args, world),
                 "window_start": {"time_us": window["time"] * 1e6, "increment": window["increment"]},
                 "gpu_launches": launches, "kernel_time_share": kernel_share,
-                "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks}
+                "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks, "arithmetic": ARITHMETIC}
     d.close()
     if rank == 0 and world == 1 and not args.no_extras and args.config == "hex":
         # the batched, the gradient and the batched-gradient workloads, timed in the same run:
@@ -852,7 +854,7 @@ def necking_line(args) -> dict:
             "agreement_vs_dual_oracle": agree,
             "gpu_launches": launches,
             "kernel_time_share": {k: round(v[0] / total_ms, 4) for k, v in prof.items()} if total_ms else None,
-            "roofline": {"bound": "fp64", "achieved": None, "peak": None, "unit": "TFLOP/s",
+            "roofline": {"bound": "fp64", "achieved": None, "peak": dynela.fp64_peak_tflops(), "unit": "TFLOP/s",
                          "frac": None, "traffic": None,
                          "kernel": "k_elem_tan<ElHex8n3D>",
                          "avg_launch_ms": tan_ms / max(tan_n, 1),

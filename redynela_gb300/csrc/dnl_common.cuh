@@ -582,7 +582,7 @@ cudaError_t copy_out(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
 // ------------------------------------------------------------------ dependent launches
 // The kernels of a step follow one another on one stream, a few microseconds each on small meshes, and
-// the gap between two plain launches costs some 2 us.  Launched by launch_next, a kernel's blocks may
+// the gap between two plain launches costs 1 to 2 us.  Launched by launch_next, a kernel's blocks may
 // become resident while its predecessor's last blocks still run; after_previous, which every such
 // kernel calls before it reads or writes anything (and before any return), waits until the
 // predecessor has completed and its writes are visible, then lets the successor's launch begin.  A

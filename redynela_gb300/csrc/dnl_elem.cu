@@ -1146,9 +1146,11 @@ __device__ __forceinline__ void elem_point(const ElemArgs &a, const Material &m,
 
 // Blocks per SM the register allocation aims at.  The pair pass of the 3D elements has instruction
 // level parallelism but long straight-line code, and waits for its instructions more than for anything
-// else: more warps hide that until the spills cost more (505,600 hexahedra: 1.93 ms unbounded at
-// 168 registers, 1.74 at 128, 1.77 at 96; 207,872 one-point hexahedra 272 us at 232, 182 at 128).  The quads
-// and the tetrahedron, and the instances with a record or general hardening, are faster unbounded.
+// else: more warps hide that until the spills cost more.  At 128 registers (four blocks), unbounded (168 and
+// 232), and 96: ten steps of 27,588 hexahedra 1.25 ms, 1.39 unbounded; the pass of 505,600 hexahedra in the
+// middle of an impact 2.06 ms, 1.91, 2.11; of 207,872 one-point hexahedra 214 us, 293, 265.  The line is drawn for
+// the meshes of usual size.  The quads and the tetrahedron, and the instances with a record or general
+// hardening, are faster unbounded.
 constexpr int elem_min_blocks(int et, bool tape, bool general)
 {
   return !tape && !general && (et == DNL_ELHEX8N3D || et == DNL_ELHEX8N3D_1PT) ? 4 : 1;

@@ -5,7 +5,7 @@
 // What bounds the FP64 pass is its ~900 FP64 instructions per hexahedral Gauss point at 64 cycles
 // each.  Here FP64 is left where its 53 bits are the point: differences of nodal coordinates and
 // displacements (exact, a few per lane) and the sums of increments into the stored state, the
-// pressure, evp, evp^n and the element forces -- about 55 instructions per point.  Everything in
+// pressure, evp and evp^n -- 29 additions per hexahedral point in the middle of an impact.  Everything in
 // between is formed as small quantities (F - I, C - I, ln U, R - I, stress increments, R X R^T - X).
 
 // element types with the pair pass (the 10-node tetrahedron's tables make its Jacobian depend on
