@@ -575,7 +575,13 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
           }
           // f = sqrt(3/2) 2 G gamma - Strial + sigma_y (the reference's terms in h cancel)
           const ff fun = ff_add(ff_sub(ff_mul(mf.dfun0, gamma), Strial), Sigv);
-          if (f_abs(fun.h) > tol * f_abs(Sigv.h)) {
+          // the residual carries some 2^-46 of the trial stress, 1e-6 of the tolerance: where that decides, FP64 does
+          const float af = f_abs(fun.h), lim = tol * f_abs(Sigv.h);
+          if (f_abs(af - lim) <= 0x1p-44f * Strial.h) {
+            bad = true;
+            break;
+          }
+          if (af > lim) {
             ff dg = ff_neg(ff_mul(fun, ff_rcp(ff_add(mf.dfun0, ff_mul(FF_CONST(kSqrt23), h)))));
             if (dg.h < 0.f && f_abs(dg.h) > gamma.h) dg = ff_mul(gamma, FF_CONST(-0.9));
             gamma = ff_add(gamma, dg);

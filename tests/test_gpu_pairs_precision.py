@@ -186,3 +186,50 @@ def test_hourglass_forces(gpu_lib):
     ah = LD(m.hourglass) * rho * c * np.cbrt(V) ** 2 / 4
     want = -ah[:, None, None] * np.einsum("eqk,eqr->ekr", g, np.einsum("eqk,ekr->eqr", g, v))
     assert _rms(got - want) <= np.sqrt(20.0) * 2.0 ** -47 * _rms(want)
+
+
+def test_radial_return_stops_where_fp64_does(gpu_lib):
+    """Trial stresses whose Newton residual, 0 or 1 iterations in, is within 1.5e-7 to 1e-6 of the stopping
+    tolerance of 1e-8: FP64 (2^-53 of the trial stress, 3e-8 of the tolerance) can tell on which side, and one
+    iteration more or less moves evp by up to 1e-11.  No increments: the trial stress is the given one."""
+    rng = np.random.default_rng(45)
+    m, x3, u3 = _elements(meshes.ELTET4N3D, 0.0, 45)
+    n = 960
+    x3, m.coords, m.conn = np.tile(x3, (20, 1)), np.tile(m.coords, (20, 1)), np.arange(4 * n).reshape(n, 4)
+    two = LD(2)
+    G2 = LD(m.young) / (1 + LD(m.poisson))
+    A, B, e = LD(m.A), LD(m.B), LD(m.n)
+    r23, r32 = np.sqrt(two / 3), np.sqrt(LD(3) / 2)
+
+    def newton(norm, evp, updates, stop=None):
+        """|f / sigma_y| and gamma after that many updates (with stop: until it is met)."""
+        h = e * B * evp ** (e - 1)
+        gamma = (norm - r23 * (A + B * evp ** e)) / (G2 * (1 + 2 * h / (3 * G2)))
+        for k in range(updates + 1):
+            x = evp + r23 * gamma
+            sigma, h = A + B * x ** e, e * B * x ** (e - 1)
+            slope = r32 * G2 + r23 * h
+            f = slope * gamma - (r32 * norm - sigma + h * r23 * gamma)
+            go = k < updates if stop is None else np.abs(f / sigma) > stop
+            gamma = np.where(go, gamma - f / slope, gamma)
+        return np.abs(f / sigma), gamma
+
+    evp = rng.uniform(1e-3, 0.3, n)
+    at = np.arange(n) % 2
+    goal = LD("1e-8") * (1 + rng.choice([-1, 1], n) * rng.uniform(1.5e-7, 1e-6, n).astype(LD))
+    lo, hi = np.full(n, LD("1e-9")), np.full(n, LD(3))
+    yield0 = (A + B * evp.astype(LD) ** e) / r32
+    for _ in range(90):
+        mid = np.sqrt(lo * hi)
+        r = np.where(at == 0, newton(yield0 * (1 + mid), evp.astype(LD), 0)[0], newton(yield0 * (1 + mid), evp.astype(LD), 1)[0])
+        lo, hi = np.where(r < goal, mid, lo), np.where(r < goal, hi, mid)
+    S = rng.normal(size=(n, 3, 3))
+    S += S.transpose(0, 2, 1)
+    S -= np.trace(S, axis1=1, axis2=2)[:, None, None] / 3 * np.eye(3)
+    S *= ((yield0 * (1 + lo)).astype(float) / np.sqrt((S * S).sum(axis=(1, 2))))[:, None, None]
+    norm = np.sqrt((S.astype(LD) ** 2).sum(axis=(1, 2)))
+    want = evp + r23 * newton(norm, evp.astype(LD), 6, LD("1e-8"))[1]
+    d = gpu_lib.GpuDomain(m)
+    d.set_state(S=S, evp=evp)
+    d.internal_forces(x3, 0.0 * x3)
+    assert np.abs(d.get_state("evp")["evp"].ravel() - want).max() <= 1e-14
