@@ -39,15 +39,14 @@ sys.path.insert(0, ROOT)
 
 from redynela_gb300 import meshes  # noqa: E402
 
-# One k_elem<ElHex8n3D> launch of the pass in pairs of FP32 numbers in the timed window of the bar cut to
-# 100 layers of elements (126,400 elements, 31,600 warps, t = 10 us, plastic impact end), from ncu:
-# dram__bytes_read.sum + dram__bytes_write.sum per element, smsp__inst_executed.sum per warp of 32 points
-# (the 400-layer bar has a smaller share of plastic points, so the issue fraction formed with it is an upper
-# bound there) and the FP64 pipe's share of its peak
+# One k_elem<ElHex8n3D> launch of the pass in pairs of FP32 numbers in the timed window (t = 10 us, plastic
+# impact end), from ncu: smsp__inst_executed.sum per warp of 32 points on this bar (126,400 warps); on the bar
+# cut to 100 layers (126,400 elements) dram__bytes_read.sum + dram__bytes_write.sum per element and the FP64
+# pipe's share of its peak
+HEX_WARP_INSTR_PER_WARP = 1351607876 / 126400
+HEX_INSTR_SOURCE = "the 505,600-element bar's timed window (t = 10 us), ncu"
 ELEM_TRAFFIC_BYTES_PER_ELEMENT = (180.76e6 + 137.80e6) / 126400
-HEX_WARP_INSTR_PER_WARP = 347404248 / 31600
 HEX_FP64_PIPE_FRAC = 0.096
-HEX_INSTR_SOURCE = "126,400 hexahedra (40 x 40 x 100 layers) in the timed window (t = 10 us), ncu"
 # what `dtype` f64 stands for: state, results and everything outside the element pass
 ARITHMETIC = ("FP64 state and results; element pass in pairs of FP32 numbers, errors at or below those of the FP64 "
               "form, which takes increments above 2^-7.75 and values out of range")
