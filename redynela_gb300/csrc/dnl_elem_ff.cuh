@@ -399,7 +399,7 @@ __device__ __forceinline__ bool elem_fast(const ElemArgs &a, const Material &m, 
   bad |= !(mg <= kFastMax) || mg * cols > kShapeMax * kFastMax * f_abs(det.h);
 
   // all of the warp's elements for the FP64 form: the rest of this pass, three quarters of it, would be for
-  // nothing (increments of 2^-5 throughout: 55,872 hexahedra 759 -> 715 us, the FP64 form alone 698; tetrahedra
+  // nothing (increments of 2^-5 throughout: 43,456 hexahedra 759 -> 715 us, the FP64 form alone 698; tetrahedra
   // 154 -> 121, 115)
   {
     const unsigned b = __ballot_sync(0xffffffffu, bad), mine = NIP > 1 ? ((1u << NIP) - 1u) << (lane - pt) : 1u << lane;
